@@ -122,78 +122,103 @@ int BitRev(int x, int bits) {
   return r;
 }
 
-// One prime's tables [W | W shoup | IW | IW shoup] in the window order of
-// the radix-16 transforms.
-template <int LOGD>
-void Permute16(const uint32_t* tab, uint32_t* t16) {
-  using N = Ntt16<LOGD>;
-  for (int w = 0; w < N::kPasses; ++w) {
-    const int m0 = 1 << N::Start(w);
-    for (int st = N::Skip(w); st < 4; ++st) {
-      for (int x = 0; x < (1 << st); ++x) {
-        for (int g = 0; g < m0; ++g) {
-          const int slot = N::Slot(w, st, x, g);
-          const int idx = (m0 << st) + (g << st) + x;
-          for (int part = 0; part < 4; ++part) {
-            t16[part * N::kD + slot] = tab[part * N::kD + idx];
-          }
-        }
-      }
+// psi^(2^j) and psi^-(2^j) mod p (j < log d) with their Shoup constants: what
+// ntt_tables_kernel multiplies up into every twiddle.
+struct RootPowers {
+  uint32_t w[kMaxPrimes][kLogMaxDegree], ws[kMaxPrimes][kLogMaxDegree];
+  uint32_t iw[kMaxPrimes][kLogMaxDegree], iws[kMaxPrimes][kLogMaxDegree];
+  uint32_t p[kMaxPrimes];
+};
+
+// Every prime's tables [W | W shoup | IW | IW shoup], W[i] = psi^brv(i), and
+// for d = 2^11..2^13 the same words in the window order of the radix-16
+// transforms (Ntt16<LOGD>::Slot) after all the plain ones. One thread per
+// twiddle pair: at most log d - 1 dependent Shoup products and two 32-bit
+// quotients, so the launch takes a few microseconds; built by the host
+// (PowMod per entry, permutation, copy) the tables took 3.2 ms at d = 4096,
+// most of every call that has a ring of its own (client, hint matrix,
+// component entry points). grid = (ceil(d / 256), kMaxPrimes).
+__global__ void ntt_tables_kernel(uint32_t* __restrict__ tables, int logd, bool with16,
+                                  RootPowers rp) {
+  const int d = 1 << logd;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= d) return;
+  const int pi = blockIdx.y;
+  const uint32_t p = rp.p[pi];
+  uint32_t w = 1, iw = 1;
+  for (int b = 0; b < logd; ++b) {
+    // Bit b of i is bit log d - 1 - b of brv(i).
+    if ((i >> b) & 1) {
+      const int j = logd - 1 - b;
+      w = shoup_mul(w, rp.w[pi][j], rp.ws[pi][j], p);
+      iw = shoup_mul(iw, rp.iw[pi][j], rp.iws[pi][j], p);
     }
   }
+  const uint32_t v[4] = {w, static_cast<uint32_t>((static_cast<uint64_t>(w) << 32) / p), iw,
+                         static_cast<uint32_t>((static_cast<uint64_t>(iw) << 32) / p)};
+  uint32_t* tab = tables + static_cast<size_t>(pi) * 4 * d;
+#pragma unroll
+  for (int part = 0; part < 4; ++part) tab[part * d + i] = v[part];
+  if (!with16) return;
+  // i = m + g' of stage j = log2 i belongs to window w, stage st of it,
+  // sub-block x and group g; entry 0 is in no stage and its place in the
+  // permuted order (the last one) stays zero.
+  uint32_t* t16 = tables + (static_cast<size_t>(kMaxPrimes) + pi) * 4 * d;
+  if (i == 0) {
+#pragma unroll
+    for (int part = 0; part < 4; ++part) t16[part * d + d - 1] = 0;
+    return;
+  }
+  const int stage = 31 - __clz(i);
+  const int passes = (logd + 3) / 4;
+  const int win = min(stage >> 2, passes - 1);
+  const int start = (win < passes - 1 || (logd & 3) == 0) ? 4 * win : logd - 4;
+  const int skip = (win == passes - 1 && (logd & 3) != 0) ? 4 - (logd & 3) : 0;
+  const int st = stage - start;
+  const int x = i & ((1 << st) - 1);
+  const int g = (i >> st) - (1 << start);
+  // Ntt16<LOGD>::Base(win) = 15 (1 + 16 + ...) = 16^win - 1.
+  const int slot = (1 << (4 * win)) - 1 + (1 << start) * ((1 << st) - (1 << skip)) +
+                   x * (1 << start) + g;
+#pragma unroll
+  for (int part = 0; part < 4; ++part) t16[part * d + slot] = v[part];
 }
 
 // Device tables for one ring degree, all primes.
 class NttTables {
  public:
-  static Status Create(int logd, std::unique_ptr<NttTables>* out) {
+  // The tables are ready for work that follows on `st`.
+  static Status Create(int logd, cudaStream_t st, std::unique_ptr<NttTables>* out) {
     if (logd < 1 || logd > kLogMaxDegree) {
       return Err(INSPIRE_INVALID_ARGUMENT, "Invalid log_d.");
     }
     std::unique_ptr<NttTables> t(new NttTables());
     t->logd_ = logd;
     const int d = 1 << logd;
-    std::vector<uint32_t> host(static_cast<size_t>(kMaxPrimes) * 4 * d);
+    RootPowers rp{};
     for (int pi = 0; pi < kMaxPrimes; ++pi) {
       const uint32_t p = kPrimes[pi];
-      const uint64_t psi = PowMod(Generator(p), (p - 1) / (2ull * d), p);
-      const uint64_t psi_inv = PowMod(psi, p - 2, p);
+      uint64_t psi = PowMod(Generator(p), (p - 1) / (2ull * d), p);
+      uint64_t psi_inv = PowMod(psi, p - 2, p);
       if (PowMod(psi, d, p) != p - 1) {
         return Err(INSPIRE_INTERNAL, "NTT root of unity check failed.");
       }
-      uint32_t* tab = host.data() + static_cast<size_t>(pi) * 4 * d;
-      for (int i = 0; i < d; ++i) {
-        const int br = BitRev(i, logd);
-        const uint32_t w = static_cast<uint32_t>(PowMod(psi, br, p));
-        const uint32_t iw = static_cast<uint32_t>(PowMod(psi_inv, br, p));
-        tab[i] = w;
-        tab[d + i] = Shoup(w, p);
-        tab[2 * d + i] = iw;
-        tab[3 * d + i] = Shoup(iw, p);
+      rp.p[pi] = p;
+      for (int j = 0; j < logd; ++j) {
+        rp.w[pi][j] = static_cast<uint32_t>(psi);
+        rp.ws[pi][j] = Shoup(rp.w[pi][j], p);
+        rp.iw[pi][j] = static_cast<uint32_t>(psi_inv);
+        rp.iws[pi][j] = Shoup(rp.iw[pi][j], p);
+        psi = psi * psi % p;
+        psi_inv = psi_inv * psi_inv % p;
       }
     }
-    if (logd >= kNtt16MinLogD && logd <= kNtt16MaxLogD) {
-      // The radix-16 order of ntt16.cuh, appended after the plain tables:
-      // W[m0 2^s + g 2^s + x] of window w at Ntt16<logd>::Slot(w, s, x, g).
-      const size_t plain = host.size();
-      host.resize(2 * plain, 0);
-      for (int pi = 0; pi < kMaxPrimes; ++pi) {
-        const uint32_t* tab = host.data() + static_cast<size_t>(pi) * 4 * d;
-        uint32_t* t16 = host.data() + plain + static_cast<size_t>(pi) * 4 * d;
-        if (logd == 11) {
-          Permute16<11>(tab, t16);
-        } else if (logd == 12) {
-          Permute16<12>(tab, t16);
-        } else {
-          Permute16<13>(tab, t16);
-        }
-      }
-      t->has16_ = true;
-    }
-    RETURN_IF_ERROR(Cuda(cudaMalloc(&t->dev_, host.size() * 4), "cudaMalloc"));
-    RETURN_IF_ERROR(Cuda(cudaMemcpy(t->dev_, host.data(), host.size() * 4,
-                                    cudaMemcpyHostToDevice),
-                         "cudaMemcpy"));
+    t->has16_ = logd >= kNtt16MinLogD && logd <= kNtt16MaxLogD;
+    const size_t words = static_cast<size_t>(kMaxPrimes) * 4 * d * (t->has16_ ? 2 : 1);
+    RETURN_IF_ERROR(Cuda(cudaMalloc(&t->dev_, words * 4), "cudaMalloc"));
+    ntt_tables_kernel<<<dim3((d + 255) / 256, kMaxPrimes), 256, 0, st>>>(t->dev_, logd,
+                                                                        t->has16_, rp);
+    RETURN_IF_ERROR(Cuda(cudaGetLastError(), "NTT tables"));
     *out = std::move(t);
     return Status{};
   }
@@ -1313,7 +1338,9 @@ Status CreateServer(const inspire_pir_params* prm, const void* db,
                   std::min(re.v_chunks * re.chunk_bits, cb)),
         &r_e));
   }
-  RETURN_IF_ERROR(NttTables::Create(prm->log_degree, &s->tables));
+  // The server's calls come on streams of their own: wait for the tables.
+  RETURN_IF_ERROR(NttTables::Create(prm->log_degree, nullptr, &s->tables));
+  RETURN_IF_ERROR(Cuda(cudaStreamSynchronize(nullptr), "NTT tables"));
   {
     int dev = 0;
     if (cudaGetDevice(&dev) == cudaSuccess) {
@@ -3144,7 +3171,7 @@ int inspire_inner_product(int32_t coeff_bits, const void* u, const void* v,
   st = PrimesFor(BoundBits(n, d, ub, vb), &r);
   if (!st.ok()) return Report(st, err, err_len);
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, &tabs);
+  st = NttTables::Create(logd, nullptr, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   NttCtx c = tabs->Ctx(r);
   const size_t total = static_cast<size_t>(n) * d;
@@ -3243,8 +3270,9 @@ int inspire_compute_hint_matrix(int32_t db_kind, int32_t coeff_bits, const void*
   int r = 0;
   Status st = PrimesFor(BoundBits(n, d, s_bits, coeff_bits), &r);
   if (!st.ok()) return Report(st, err, err_len);
+  const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, &tabs);
+  st = NttTables::Create(logd, cs, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   NttCtx c = tabs->Ctx(r);
   int dev = 0, sms = 152;
@@ -3283,7 +3311,6 @@ int inspire_compute_hint_matrix(int32_t db_kind, int32_t coeff_bits, const void*
       }
     }
   }
-  const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   DevBuf dv, dV, dres, ddb, dout;
   st = dv.Upload(vinv.data(), vinv.size());
   if (st.ok()) st = dV.Alloc(static_cast<size_t>(n) * r * d * 4);
@@ -3374,7 +3401,7 @@ int inspire_external_product(const inspire_pir_params* params,
                  &r);
   if (!st.ok()) return Report(st, err, err_len);
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(params->log_degree, &tabs);
+  st = NttTables::Create(params->log_degree, nullptr, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   NttCtx c = tabs->Ctx(r);
   const size_t w = cb / 8;
@@ -3473,11 +3500,11 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
   const size_t w = coeff_bits / 8;
   const size_t chain_smem = d * w + static_cast<size_t>(d) * 4 * (1 + r);
   if (chain_smem > 227 * 1024) return fail("ring degree and gadget too large.");
+  const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, &tabs);
+  st = NttTables::Create(logd, cs, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   const NttCtx c = tabs->Ctx(r);
-  const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   const size_t mw = elem_size(mat_kind);
   const size_t dd = static_cast<size_t>(d) * d;
   const int64_t chain_stride = static_cast<int64_t>(d / 2 - 1) * k * d;
@@ -3701,11 +3728,11 @@ int inspire_client_create_requests(const inspire_pir_params* params,
   int r = 0;
   Status st = PrimesFor(BoundBits(1, d, cb, 2), &r);
   if (!st.ok()) return Report(st, err, err_len);
+  const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, &tabs);
+  st = NttTables::Create(logd, cs, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   const NttCtx c = tabs->Ctx(r);
-  const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   const size_t w = cb / 8;
   DevBuf dkeys, da, didx, dshat, dfd, dsd, dpk;
   const int8_t* keys = secret_keys;
@@ -3793,11 +3820,11 @@ int inspire_client_process_responses(const inspire_pir_params* params,
   int r = 0;
   Status st = PrimesFor(BoundBits(1, d, cb, 2), &r);
   if (!st.ok()) return Report(st, err, err_len);
+  const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, &tabs);
+  st = NttTables::Create(logd, cs, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   const NttCtx c = tabs->Ctx(r);
-  const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   const size_t w = cb / 8;
   DevBuf dkeys, dresp, dout, dshat;
   const int8_t* keys = secret_keys;
@@ -3865,7 +3892,7 @@ int inspire_finalize_matrix_pack(const inspire_pir_params* params,
                  &r);
   if (!st.ok()) return Report(st, err, err_len);
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(params->log_degree, &tabs);
+  st = NttTables::Create(params->log_degree, nullptr, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   NttCtx c = tabs->Ctx(r);
   const size_t w = cb / 8;
