@@ -318,9 +318,20 @@ cudaError_t launch_typed(const void* db, int64_t db_cols, const void* q1,
         blocks, db, db_cols, q1, q1_stride, pk, pk_cols, yg, yg_stride, out, out_stride, rows,
         stream);
   } else {
-    constexpr int RB = NQ >= 4 ? 2 : 4;
-    return launch_rows<T, DbT, MatT, RB, NQ, kThreads, false>(
-        (rows + RB - 1) / RB, db, db_cols, q1, q1_stride, pk, pk_cols, yg, yg_stride, out,
+    // Rows per block. A thread's query loads (NQ x 32 bytes of u32 words per
+    // 16-byte u16 vector, from L1) are shared by the block's rows: with two
+    // rows they take 40 of the 43 cycles in which HBM delivers a warp's 1 KB of
+    // matrix at NQ = 4, so three or four queries take four rows too (4 queries
+    // at 32768 x 32768 u16 + 32768 x 8192 i32 over Z_2^32: 728 -> 635 us).
+    // Below 8192 rows the blocks would fill the device barely twice and two
+    // rows stay ahead (4096 rows over Z_2^64: 58 against 62 us).
+    if (NQ >= 3 && rows < 8192) {
+      return launch_rows<T, DbT, MatT, 2, NQ, kThreads, false>(
+          (rows + 1) / 2, db, db_cols, q1, q1_stride, pk, pk_cols, yg, yg_stride, out,
+          out_stride, rows, stream);
+    }
+    return launch_rows<T, DbT, MatT, 4, NQ, kThreads, false>(
+        (rows + 3) / 4, db, db_cols, q1, q1_stride, pk, pk_cols, yg, yg_stride, out,
         out_stride, rows, stream);
   }
 }
@@ -330,7 +341,12 @@ cudaError_t launch_nq(int nq, const void* db, int64_t db_cols, const void* q1,
                       int64_t q1_stride, const void* pk, int64_t pk_cols,
                       const void* yg, int64_t yg_stride, void* out,
                       int64_t out_stride, int64_t rows, cudaStream_t stream) {
-  // Split the batch into groups of 4, 2 and 1 queries.
+  // Split the batch into groups of 4, then one group of the 1 to 3 left: each
+  // group is one pass over the matrices. Over Z_2^64 three requests go as 2 + 1:
+  // the 64-bit multiply-adds bound them, and the group of three (its 24 sums
+  // of 64 bits a thread) took 425 us against 374 at 16384 x 16384 u16 +
+  // 16384 x 4096 i32; over Z_2^32 one pass took 590 us against 940 at
+  // 32768 x 32768 u16 + 32768 x 8192 i32.
   int done = 0;
   cudaError_t e = cudaSuccess;
   auto off_q = [&](const void* p, int64_t stride, int q) -> const void* {
@@ -346,6 +362,12 @@ cudaError_t launch_nq(int nq, const void* db, int64_t db_cols, const void* q1,
       e = launch_typed<T, DbT, MatT, 4>(db, db_cols, a, q1_stride, pk, pk_cols, b,
                                         yg_stride, o, out_stride, rows, stream);
       done += 4;
+    } else if (left == 3 && sizeof(T) == 4) {
+      if constexpr (sizeof(T) == 4) {
+        e = launch_typed<T, DbT, MatT, 3>(db, db_cols, a, q1_stride, pk, pk_cols, b,
+                                          yg_stride, o, out_stride, rows, stream);
+      }
+      done += 3;
     } else if (left >= 2) {
       e = launch_typed<T, DbT, MatT, 2>(db, db_cols, a, q1_stride, pk, pk_cols, b,
                                         yg_stride, o, out_stride, rows, stream);
