@@ -62,13 +62,6 @@ __device__ __forceinline__ uint32_t mont_mul(uint32_t a, uint32_t b,
 // conditional subtraction in two instructions.
 __device__ __forceinline__ uint32_t umin32(uint32_t a, uint32_t b) { return min(a, b); }
 
-__device__ __forceinline__ uint32_t reduce_u32(uint32_t x, uint32_t p) {
-  // x < 2^32 < 3p for p > 2^31 / 1.5
-  if (x >= p) x -= p;
-  if (x >= p) x -= p;
-  return x;
-}
-
 // Shoup without the final correction: a * w mod p in [0, 2p) for any
 // 32-bit a and a constant w < p with ws = floor(w * 2^32 / p).
 __device__ __forceinline__ uint32_t shoup_mul_lazy(uint32_t a, uint32_t w,
@@ -76,8 +69,17 @@ __device__ __forceinline__ uint32_t shoup_mul_lazy(uint32_t a, uint32_t w,
   return a * w - __umulhi(a, ws) * p;
 }
 
-__device__ __forceinline__ uint32_t reduce_u64(uint64_t x, uint32_t p) {
-  return static_cast<uint32_t>(x % p);
+// x mod p in [0, 2p) for any 32-bit x, with one_s = floor(2^32 / p): the
+// Shoup product by 1.
+__device__ __forceinline__ uint32_t barrett_lazy(uint32_t x, uint32_t one_s, uint32_t p) {
+  return x - __umulhi(x, one_s) * p;
+}
+
+// Signed Montgomery without the final correction: a * b * 2^-32 mod p in
+// (0, 2p), for a b < 2^32 p.
+__device__ __forceinline__ uint32_t mont_mul_lazy(uint32_t a, uint32_t b, uint32_t p,
+                                                  uint32_t pinv) {
+  return __umulhi(a, b) - __umulhi(a * b * pinv, p) + p;
 }
 #endif
 

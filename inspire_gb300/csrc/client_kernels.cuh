@@ -118,11 +118,7 @@ __device__ __forceinline__ void cl_times_key(const T* a, const uint32_t* s_hat, 
     uint32_t* x = sm + static_cast<int64_t>(pi) * d;
     const uint32_t p = c.p[pi];
     for (int j = threadIdx.x; j < d; j += blockDim.x) {
-      if constexpr (sizeof(T) == 4) {
-        x[j] = reduce_u32(a[j], p);
-      } else {
-        x[j] = reduce_u64(a[j], p);
-      }
+      x[j] = reduce_word(a[j], c, pi);
     }
     ntt_forward_t<ITERS>(x, c, pi);
     const uint32_t* sh = s_hat + static_cast<int64_t>(pi) * d;

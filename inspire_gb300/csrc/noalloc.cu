@@ -197,6 +197,9 @@ const DegreeConsts& ConstsFor(int logd) {
       const uint64_t r32 = (1ull << 32) % p;
       c.scale[i] = static_cast<uint32_t>(pow_mod(d, p - 2, p) * r32 % p);
       c.scale_s[i] = shoup_of(c.scale[i], p);
+      c.one_s[i] = static_cast<uint32_t>((1ull << 32) / p);
+      c.r32[i] = static_cast<uint32_t>(r32);
+      c.r32_s[i] = shoup_of(c.r32[i], p);
       uint64_t prod = 1;
       for (int j = 0; j < i; ++j) prod *= kNoAllocPrimes[j];
       c.pm[i] = prod;

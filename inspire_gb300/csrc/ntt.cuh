@@ -23,13 +23,33 @@ struct NttCtx {
   uint32_t scale_s[kMaxPrimes];  // the 2^-32 of the Montgomery pointwise step
   uint32_t garner[kMaxPrimes][kMaxPrimes];  // [j][i] = p_j^-1 * 2^32 mod p_i
   uint64_t pm[kMaxPrimes];                  // prod_{j<i} p_j mod 2^64
+  // Reductions of wide words: floor(2^32 / p), and 2^32 mod p with its Shoup
+  // constant.
+  uint32_t one_s[kMaxPrimes];
+  uint32_t r32[kMaxPrimes];
+  uint32_t r32_s[kMaxPrimes];
   const uint32_t* tables;  // [prime][4][d]: psi_rev, shoup, ipsi_rev, shoup
-  // The same tables permuted for the radix-16 transform of ntt16.cuh
-  // ([prime][4][d]); null unless d = 4096.
-  const uint32_t* tables16;
+  // The twiddles as (value, Shoup constant) pairs in the order of the radix-16
+  // transforms of ntt16.cuh, [prime][forward, inverse][d]; null unless
+  // d = 2048..8192 and the primes are below 2^27.
+  const uint2* tables16;
 };
 
 #ifdef __CUDACC__
+// x mod p_pi in [0, p) for a full word.
+__device__ __forceinline__ uint32_t reduce_word(uint32_t x, const NttCtx& c, int pi) {
+  const uint32_t p = c.p[pi];
+  const uint32_t r = barrett_lazy(x, c.one_s[pi], p);
+  return umin32(r, r - p);
+}
+__device__ __forceinline__ uint32_t reduce_word(uint64_t x, const NttCtx& c, int pi) {
+  const uint32_t p = c.p[pi];
+  const uint32_t h =
+      shoup_mul(static_cast<uint32_t>(x >> 32), c.r32[pi], c.r32_s[pi], p);
+  const uint32_t s = h + reduce_word(static_cast<uint32_t>(x), c, pi);
+  return umin32(s, s - p);
+}
+
 // Forward transform. Two Cooley-Tukey stages at a time: the quad
 // (x0, x1, x2, x3) = a[j], a[j+t/2], a[j+t], a[j+3t/2] takes stage (m, t)
 // with twiddle W[m+i] on (x0,x2),(x1,x3), then stage (2m, t/2) with W[2m+2i]
@@ -283,6 +303,32 @@ __device__ __forceinline__ void ntt_inverse_t(uint32_t* a, const NttCtx& c,
 // Garner reconstruction: x[i] < p_i -> the integer in
 // [-(p_{r-1}-1)/2 * P', (p_{r-1}+1)/2 * P') (P' = product of the other
 // primes) congruent to x, reduced mod 2^w.
+// The same for R primes known at compile time (a third of the code).
+template <typename T, int R>
+__device__ __forceinline__ T crt_fixed(const uint32_t (&x)[R], const NttCtx& c) {
+  uint32_t a[R];
+  a[0] = x[0];
+#pragma unroll
+  for (int i = 1; i < R; ++i) {
+    const uint32_t p = c.p[i];
+    uint32_t v = x[i];
+#pragma unroll
+    for (int j = 0; j < i; ++j) {
+      const uint32_t aj = umin32(a[j], a[j] - p);
+      v = mont_mul(umin32(v - aj, v - aj + p), c.garner[j][i], p, c.pinv[i]);
+    }
+    a[i] = v;
+  }
+  // A top digit above the half counts as negative.
+  T acc = static_cast<T>(a[R - 1]) * static_cast<T>(c.pm[R - 1]);
+  if (a[R - 1] > c.half[R - 1]) {
+    acc -= static_cast<T>(c.p[R - 1]) * static_cast<T>(c.pm[R - 1]);
+  }
+#pragma unroll
+  for (int i = 0; i + 1 < R; ++i) acc += static_cast<T>(a[i]) * static_cast<T>(c.pm[i]);
+  return acc;
+}
+
 template <typename T>
 __device__ __forceinline__ T crt_reconstruct(const uint32_t (&x)[kMaxPrimes],
                                              const NttCtx& c) {

@@ -16,10 +16,21 @@
 // order, coalesced), the last one e_k = 16 tid + k. Stage s of a window
 // pairs k with k + 8 / 2^s and takes W[m0 2^s + g 2^s + (k >> (4 - s))].
 //
-// Twiddles are read from a permuted copy of the tables (built on the host):
-// window w, stage s, sub-block x, group g at base_w + m0 (2^s - 2^skip) +
-// x m0 + g, so the threads of a warp read one word, a few words or
-// consecutive words.
+// Twiddles are read as (value, Shoup constant) pairs from a permuted copy of
+// the tables (ntt_tables_kernel): window w, stage s, sub-block x, group g at
+// base_w + m0 (2^s - 2^skip) + x m0 + g, so the threads of a warp read one
+// pair, a few pairs or consecutive pairs.
+//
+// The primes are below 2^27, so 32 p < 2^32 and the butterflies reduce
+// nothing (after Harvey, "Faster arithmetic for number-theoretic transforms",
+// 2014, whose [0, 4p) this stretches): a forward butterfly is Shoup's product
+// without its correction (three multiplier instructions, four of the 64
+// lanes per cycle that a multiplier takes, since the high product counts
+// twice), u + v and u - v + 2p, and a value grows by at most 2p per stage.
+// An inverse butterfly doubles the bound of its sum, so every window of four
+// stages ends with one reduction of the values above 2p. With 31-bit primes
+// the same butterfly took four more instructions and the transforms were
+// bound by issue; the multiplier is the bound now.
 //
 // Shared memory holds coefficient e at e ^ swz(e >> 5), with a swz per size
 // that keeps every pass's access pattern free of bank conflicts (the
@@ -96,10 +107,10 @@ __device__ __forceinline__ void ntt16_sync(int bar) {
   }
 }
 
-// A twiddle word: read-only global memory (kSmem = false) or a copy of the
+// A twiddle pair: read-only global memory (kSmem = false) or a copy of the
 // tables in shared memory.
 template <bool kSmem>
-__device__ __forceinline__ uint32_t ntt16_tw(const uint32_t* t, int i) {
+__device__ __forceinline__ uint2 ntt16_tw(const uint2* t, int i) {
   if constexpr (kSmem) {
     return t[i];
   } else {
@@ -107,168 +118,190 @@ __device__ __forceinline__ uint32_t ntt16_tw(const uint32_t* t, int i) {
   }
 }
 
+// Before the inverse stage of half-length h = 2^L (stages 1, 2, .. 2^(L-1)
+// done on values below 2p), coefficient k holds less than 2p << grow(k, L):
+// its bound doubled in each stage since it last came out of a product.
+__host__ __device__ constexpr int ntt16_grow(int k, int L) {
+  const int i = k & ((1 << L) - 1);
+  if (i == 0) return L;
+  int hb = 0;
+  while ((i >> (hb + 1)) != 0) ++hb;
+  return L - 1 - hb;
+}
+
 // The stages of window w on the thread's 16 coefficients, forward (Cooley-
 // Tukey, stages skip .. 3) or inverse (Gentleman-Sande, 3 .. skip). With a
 // compile-time window every index folds; the compact transforms pass a
-// run-time one and the same instructions serve every window.
-//
-// Values stay in [0, 2p) between butterflies (2p < 2^32 for the 31-bit
-// primes): each butterfly brings its two inputs to [0, p) with one unsigned
-// min each, forms u + v and u - v + p in [0, 2p) without a compare, and the
-// twiddle product is Shoup's without its correction (Harvey, "Faster
-// arithmetic for number-theoretic transforms", 2014, with the reductions
-// moved to the inputs since 4p does not fit 32 bits). ntt16_forward and
-// ntt16_inverse_tw reduce to [0, p) at the end unless asked not to.
+// run-time one and the same instructions serve every window. Forward: adds
+// less than 2p per stage to values of any size below 2^32. Inverse: from
+// values below 2p to values below 32p.
 template <int LOGD, bool kSmem, bool kInverse>
-__device__ __forceinline__ void ntt16_window(uint32_t (&x)[16],
-                                             const uint32_t* __restrict__ tw,
-                                             const uint32_t* __restrict__ tws,
+__device__ __forceinline__ void ntt16_window(uint32_t (&x)[16], const uint2* __restrict__ tw,
                                              uint32_t p, int w, int g) {
   const int m0 = 1 << Ntt16<LOGD>::Start(w);
   const int skip = Ntt16<LOGD>::Skip(w);
   const int base = Ntt16<LOGD>::Base(w) + g - m0 * (1 << skip);
+  const uint32_t p2 = 2 * p;
 #pragma unroll
   for (int si = 0; si < 4; ++si) {
     const int s = kInverse ? 3 - si : si;
     if (s < skip) continue;
     const int half = 8 >> s;
-    uint32_t wv[8], wsv[8];
+    uint2 wv[8];
 #pragma unroll
-    for (int b = 0; b < (1 << s); ++b) {
-      const int slot = base + m0 * ((1 << s) + b);
-      wv[b] = ntt16_tw<kSmem>(tw, slot);
-      wsv[b] = ntt16_tw<kSmem>(tws, slot);
-    }
+    for (int b = 0; b < (1 << s); ++b) wv[b] = ntt16_tw<kSmem>(tw, base + m0 * ((1 << s) + b));
 #pragma unroll
     for (int b = 0; b < (1 << s); ++b) {
 #pragma unroll
       for (int i = 0; i < half; ++i) {
         const int k = b * 2 * half + i;
+        const uint32_t u = x[k], v = x[k + half];
         if (kInverse) {
-          const uint32_t u = umin32(x[k], x[k] - p);
-          const uint32_t v = umin32(x[k + half], x[k + half] - p);
           x[k] = u + v;
-          x[k + half] = shoup_mul_lazy(u + p - v, wv[b], wsv[b], p);
+          x[k + half] =
+              shoup_mul_lazy(u - v + (p2 << ntt16_grow(i, 3 - s)), wv[b].x, wv[b].y, p);
         } else {
-          const uint32_t u = umin32(x[k], x[k] - p);
-          uint32_t v = shoup_mul_lazy(x[k + half], wv[b], wsv[b], p);
-          v = umin32(v, v - p);
-          x[k] = u + v;
-          x[k + half] = u + p - v;
+          const uint32_t y = shoup_mul_lazy(v, wv[b].x, wv[b].y, p);
+          x[k] = u + y;
+          x[k + half] = u - y + p2;
         }
       }
     }
   }
 }
 
+// How far coefficient k of window w's inverse result may be above 2p (below
+// 2p << n); with w < 0 the largest over the windows that another one follows.
+template <int LOGD>
+__host__ __device__ constexpr int ntt16_excess(int k, int w) {
+  if (w >= 0) return ntt16_grow(k, 4 - Ntt16<LOGD>::Skip(w));
+  int n = 0;
+  for (int v = 1; v < Ntt16<LOGD>::kPasses; ++v) {
+    const int e = ntt16_grow(k, 4 - Ntt16<LOGD>::Skip(v));
+    n = e > n ? e : n;
+  }
+  return n;
+}
+
+// Between two inverse windows: back below 2p.
+template <int LOGD>
+__device__ __forceinline__ void ntt16_settle(uint32_t (&x)[16], uint32_t p, uint32_t one_s,
+                                             int w) {
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    const int n = ntt16_excess<LOGD>(k, w);
+    if (n >= 2) {
+      x[k] = barrett_lazy(x[k], one_s, p);
+    } else if (n == 1) {
+      x[k] = umin32(x[k], x[k] - 2 * p);
+    }
+  }
+}
+
+// Byte offset in a d-word buffer of the thread's coefficient k of window w.
+// The swizzle is linear over GF(2) and the bits of stride * k are apart from
+// those of the base, so the 16 offsets are one base XOR sums of four words:
+// a few instructions where a general position took eight per coefficient,
+// most of a compact pass's code.
+template <int LOGD>
+struct Ntt16Slots {
+  uint32_t base, bit[4];
+  __device__ __forceinline__ Ntt16Slots(int w, int tid) {
+    int e, stride, g;
+    ntt16_geometry<LOGD>(w, tid, e, stride, g);
+    base = 4u * ntt16_pos<LOGD>(e);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) bit[i] = 4u * ntt16_pos<LOGD>(stride << i);
+  }
+  __device__ __forceinline__ uint32_t operator()(int k) const {
+    return base ^ ((k & 1) ? bit[0] : 0u) ^ ((k & 2) ? bit[1] : 0u) ^ ((k & 4) ? bit[2] : 0u) ^
+           ((k & 8) ? bit[3] : 0u);
+  }
+};
+
 template <int LOGD>
 __device__ __forceinline__ void ntt16_store(const uint32_t (&x)[16], uint32_t* xs, int w,
                                             int tid) {
-  int base, stride, g;
-  ntt16_geometry<LOGD>(w, tid, base, stride, g);
+  const Ntt16Slots<LOGD> at(w, tid);
+  char* b = reinterpret_cast<char*>(xs);
 #pragma unroll
-  for (int k = 0; k < 16; ++k) xs[ntt16_pos<LOGD>(base + stride * k)] = x[k];
+  for (int k = 0; k < 16; ++k) *reinterpret_cast<uint32_t*>(b + at(k)) = x[k];
 }
 
 template <int LOGD>
 __device__ __forceinline__ void ntt16_load(uint32_t (&x)[16], const uint32_t* xs, int w,
                                            int tid) {
-  int base, stride, g;
-  ntt16_geometry<LOGD>(w, tid, base, stride, g);
+  const Ntt16Slots<LOGD> at(w, tid);
+  const char* b = reinterpret_cast<const char*>(xs);
 #pragma unroll
-  for (int k = 0; k < 16; ++k) x[k] = xs[ntt16_pos<LOGD>(base + stride * k)];
+  for (int k = 0; k < 16; ++k) x[k] = *reinterpret_cast<const uint32_t*>(b + at(k));
 }
 
 // Forward transform. In: x[k] = coefficient tid + (d / 16) k, any value
-// below 2p. Out: x[k] = NTT slot 16 tid + k in [0, p) (the bit-reversed
-// output array of ntt_forward). `xs`
-// is a d-word shared buffer, free again when this returns. tab16 = the
-// prime's permuted tables [W | W shoup | IW | IW shoup], d words each. tid
-// in [0, d / 16) within the group that synchronises on `bar`. kSmem: the
-// tables were copied to shared memory (tab16 points there). kCompact: one
-// window body for all windows (a third of the code, for launches whose
-// blocks each run once per SM, where fetching unrolled code sets the time).
-// kLazyOut: the slots are left in [0, 2p), for a caller that only passes
-// them to mont_mul with a reduced second operand (a b < 2 p^2 < 2^32 p).
-template <int LOGD, bool kSmem = false, bool kCompact = false, bool kLazyOut = false>
+// below 6p. Out: x[k] = NTT slot 16 tid + k (the bit-reversed output array of
+// ntt_forward) below 32p, fit for a Montgomery product with a factor below p;
+// reduced to [0, p) with kReduce. `xs` is a d-word shared buffer, free again
+// when this returns. tw = the prime's forward pairs. tid in [0, d / 16) within
+// the group that synchronises on `bar`. kSmem: the pairs were copied to
+// shared memory. kCompact: one window body for all windows (a third of the
+// code, for launches whose blocks each run once per SM, where fetching
+// unrolled code sets the time).
+template <int LOGD, bool kSmem = false, bool kCompact = false, bool kReduce = false>
 __device__ __forceinline__ void ntt16_forward(uint32_t (&x)[16], uint32_t* xs,
-                                              const uint32_t* __restrict__ tab16,
-                                              uint32_t p, int tid, int bar = 0) {
+                                              const uint2* __restrict__ tw, uint32_t p,
+                                              uint32_t one_s, int tid, int bar = 0) {
   using N = Ntt16<LOGD>;
-  const uint32_t* tw = tab16;
-  const uint32_t* tws = tab16 + N::kD;
+  auto pass = [&](int w) {
+    int base, stride, g;
+    ntt16_geometry<LOGD>(w, tid, base, stride, g);
+    if (w > 0) ntt16_load<LOGD>(x, xs, w, tid);
+    ntt16_window<LOGD, kSmem, false>(x, tw, p, w, g);
+    // The store goes to the words this thread read (no barrier between).
+    if (w < N::kPasses - 1) ntt16_store<LOGD>(x, xs, w, tid);
+    ntt16_sync<LOGD>(bar);
+  };
   if constexpr (kCompact) {
 #pragma unroll 1
-    for (int w = 0; w < N::kPasses; ++w) {
-      int base, stride, g;
-      ntt16_geometry<LOGD>(w, tid, base, stride, g);
-      if (w > 0) ntt16_load<LOGD>(x, xs, w, tid);
-      ntt16_window<LOGD, kSmem, false>(x, tw, tws, p, w, g);
-      if (w < N::kPasses - 1) ntt16_store<LOGD>(x, xs, w, tid);
-      ntt16_sync<LOGD>(bar);
-    }
+    for (int w = 0; w < N::kPasses; ++w) pass(w);
   } else {
 #pragma unroll
-    for (int w = 0; w < N::kPasses; ++w) {
-      int base, stride, g;
-      ntt16_geometry<LOGD>(w, tid, base, stride, g);
-      if (w > 0) ntt16_load<LOGD>(x, xs, w, tid);
-      ntt16_window<LOGD, kSmem, false>(x, tw, tws, p, w, g);
-      // The store goes to the words this thread read (no barrier between).
-      if (w < N::kPasses - 1) ntt16_store<LOGD>(x, xs, w, tid);
-      ntt16_sync<LOGD>(bar);
-    }
+    for (int w = 0; w < N::kPasses; ++w) pass(w);
   }
-  if constexpr (!kLazyOut) {
-    // [0, 2p) -> [0, p).
+  if constexpr (kReduce) {
 #pragma unroll
-    for (int k = 0; k < 16; ++k) x[k] = umin32(x[k], x[k] - p);
+    for (int k = 0; k < 16; ++k) {
+      const uint32_t r = barrett_lazy(x[k], one_s, p);
+      x[k] = umin32(r, r - p);
+    }
   }
 }
 
-// Inverse transform without the 1/d scaling. In: x[k] = slot 16 tid + k,
-// any value below 2p. Out: x[k] = coefficient tid + (d / 16) k in [0, p).
-// itw / itws: the permuted
-// inverse twiddles and their Shoup constants.
-template <int LOGD, bool kSmem = false, bool kCompact = false>
-__device__ __forceinline__ void ntt16_inverse_tw(uint32_t (&x)[16], uint32_t* xs,
-                                                 const uint32_t* __restrict__ itw,
-                                                 const uint32_t* __restrict__ itws,
-                                                 uint32_t p, int tid, int bar = 0) {
-  using N = Ntt16<LOGD>;
-  if constexpr (kCompact) {
-#pragma unroll 1
-    for (int w = N::kPasses - 1; w >= 0; --w) {
-      int base, stride, g;
-      ntt16_geometry<LOGD>(w, tid, base, stride, g);
-      if (w < N::kPasses - 1) ntt16_load<LOGD>(x, xs, w, tid);
-      ntt16_window<LOGD, kSmem, true>(x, itw, itws, p, w, g);
-      if (w > 0) ntt16_store<LOGD>(x, xs, w, tid);
-      ntt16_sync<LOGD>(bar);
-    }
-  } else {
-#pragma unroll
-    for (int w = N::kPasses - 1; w >= 0; --w) {
-      int base, stride, g;
-      ntt16_geometry<LOGD>(w, tid, base, stride, g);
-      if (w < N::kPasses - 1) ntt16_load<LOGD>(x, xs, w, tid);
-      ntt16_window<LOGD, kSmem, true>(x, itw, itws, p, w, g);
-      if (w > 0) ntt16_store<LOGD>(x, xs, w, tid);
-      ntt16_sync<LOGD>(bar);
-    }
-  }
-  // [0, 2p) -> [0, p).
-#pragma unroll
-  for (int k = 0; k < 16; ++k) x[k] = umin32(x[k], x[k] - p);
-}
-
-// The inverse with the prime's whole table block [W | W shoup | IW | IW shoup].
+// Inverse transform without the 1/d scaling. In: x[k] = slot 16 tid + k below
+// 2p. Out: x[k] = coefficient tid + (d / 16) k below 32p (the scaling's Shoup
+// product takes any word). itw = the prime's inverse pairs.
 template <int LOGD, bool kSmem = false, bool kCompact = false>
 __device__ __forceinline__ void ntt16_inverse(uint32_t (&x)[16], uint32_t* xs,
-                                              const uint32_t* __restrict__ tab16,
-                                              uint32_t p, int tid, int bar = 0) {
-  ntt16_inverse_tw<LOGD, kSmem, kCompact>(x, xs, tab16 + 2 * Ntt16<LOGD>::kD,
-                                          tab16 + 3 * Ntt16<LOGD>::kD, p, tid, bar);
+                                              const uint2* __restrict__ itw, uint32_t p,
+                                              uint32_t one_s, int tid, int bar = 0) {
+  using N = Ntt16<LOGD>;
+  auto pass = [&](int w) {
+    int base, stride, g;
+    ntt16_geometry<LOGD>(w, tid, base, stride, g);
+    if (w < N::kPasses - 1) ntt16_load<LOGD>(x, xs, w, tid);
+    ntt16_window<LOGD, kSmem, true>(x, itw, p, w, g);
+    if (w > 0) {
+      ntt16_settle<LOGD>(x, p, one_s, kCompact ? -1 : w);
+      ntt16_store<LOGD>(x, xs, w, tid);
+    }
+    ntt16_sync<LOGD>(bar);
+  };
+  if constexpr (kCompact) {
+#pragma unroll 1
+    for (int w = N::kPasses - 1; w >= 0; --w) pass(w);
+  } else {
+#pragma unroll
+    for (int w = N::kPasses - 1; w >= 0; --w) pass(w);
+  }
 }
 
 // The slot layout the forward transform leaves (x[k] = slot 16 tid + k) in

@@ -58,15 +58,6 @@ __device__ __forceinline__ T rescale_word(T c, int lcur, int lnew) {
   return (c >> s) + ((c >> (s - 1)) & T{1});
 }
 
-template <typename T>
-__device__ __forceinline__ uint32_t to_residue(T x, uint32_t p) {
-  if constexpr (sizeof(T) == 4) {
-    return reduce_u32(x, p);
-  } else {
-    return reduce_u64(x, p);
-  }
-}
-
 // Gadget digit `dg` of a LowBits'd coefficient (Polynomial::GadgetInv with
 // the rounding shift when log_modulus > digits * log_digit).
 template <typename T>
@@ -97,7 +88,7 @@ ntt_coeffs_kernel(const T* __restrict__ src, int64_t src_qstride,
   const uint32_t p = c.p[pi];
   const T* in = src + q * src_qstride + src_off + poly * poly_stride;
   for (int j = threadIdx.x; j < d; j += blockDim.x) {
-    smem[j] = to_residue<T>(in[j] & mask, p);
+    smem[j] = reduce_word(static_cast<T>(in[j] & mask), c, pi);
   }
   ntt_forward_t<ITERS>(smem, c, pi);
   uint32_t* out = dst + ((static_cast<int64_t>(q) * npoly + poly) * c.r + pi) * d;
@@ -126,8 +117,9 @@ ntt_coeffs16_kernel(const T* __restrict__ src, int64_t src_qstride,
     const uint32_t p = c.p[pi];
     uint32_t x[16];
 #pragma unroll
-    for (int k = 0; k < 16; ++k) x[k] = to_residue<T>(v[k], p);
-    ntt16_forward<LOGD>(x, xs, c.tables16 + static_cast<size_t>(pi) * 4 * d, p, tid);
+    for (int k = 0; k < 16; ++k) x[k] = reduce_word(v[k], c, pi);
+    ntt16_forward<LOGD, false, false, true>(
+        x, xs, c.tables16 + static_cast<size_t>(pi) * 2 * d, p, c.one_s[pi], tid);
     uint4* out = reinterpret_cast<uint4*>(
         dst + ((static_cast<int64_t>(q) * npoly + poly) * c.r + pi) * d + 16 * tid);
 #pragma unroll
@@ -280,7 +272,8 @@ finalize16_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restrict__ 
         acc[4 * w + 3] = add_mod(acc[4 * w + 3], mont_mul(a.w, b.w, p, pinv), p);
       }
     }
-    ntt16_inverse<LOGD>(acc, xs, c.tables16 + static_cast<size_t>(pi) * 4 * d, p, tid);
+    ntt16_inverse<LOGD>(acc, xs, c.tables16 + static_cast<size_t>(2 * pi + 1) * d, p,
+                        c.one_s[pi], tid);
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       res[pi * d + tid + NT * j] = shoup_mul(acc[j], c.scale[pi], c.scale_s[pi], p);
@@ -323,7 +316,7 @@ finalize16_pair_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restri
   const int lt = tid & (NT - 1);
   const int bar = 1 + grp;
   uint32_t* xs = smem + grp * d;
-  uint32_t* itab = smem + NGR * d + grp * 2 * d;  // IW | IW shoup of the prime
+  uint32_t* itab = smem + NGR * d + grp * 2 * d;  // the prime's inverse pairs
   uint32_t* res = smem + 3 * NGR * d;             // [r][d] scaled residues
   const int s = blockIdx.x;
   const int q = blockIdx.y;
@@ -331,7 +324,7 @@ finalize16_pair_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restri
     const uint32_t p = c.p[pi];
     const uint32_t pinv = c.pinv[pi];
     const uint4* g16 = reinterpret_cast<const uint4*>(
-        c.tables16 + static_cast<size_t>(pi) * 4 * d + 2 * d);
+        c.tables16 + static_cast<size_t>(2 * pi + 1) * d);
     uint4* s16 = reinterpret_cast<uint4*>(itab);
 #pragma unroll
     for (int i = 0; i < 2 * d / 4 / NT; ++i) {
@@ -355,7 +348,8 @@ finalize16_pair_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restri
       }
     }
     ntt16_sync<LOGD>(bar);  // the group's copy of the tables is complete
-    ntt16_inverse_tw<LOGD, true, true>(acc, xs, itab, itab + d, p, lt, bar);
+    ntt16_inverse<LOGD, true, true>(acc, xs, reinterpret_cast<const uint2*>(itab), p,
+                                    c.one_s[pi], lt, bar);
 #pragma unroll
     for (int j = 0; j < 16; ++j) {
       res[pi * d + lt + NT * j] = shoup_mul(acc[j], c.scale[pi], c.scale_s[pi], p);
@@ -419,7 +413,7 @@ hint_rows_kernel(const S* __restrict__ db, int64_t cols, int n,
   for (int k = 0; k < n; ++k) {
     __syncthreads();
     for (int j = threadIdx.x; j < d; j += blockDim.x) {
-      smem[j] = reduce_u32(static_cast<uint32_t>(src[static_cast<int64_t>(k) * d + j]), p);
+      smem[j] = reduce_word(static_cast<uint32_t>(src[static_cast<int64_t>(k) * d + j]), c, pi);
     }
     ntt_forward_t<ITERS>(smem, c, pi);
     const uint32_t* vk = V + (static_cast<int64_t>(k) * c.r + pi) * d;
@@ -445,7 +439,7 @@ hint_rows_kernel(const S* __restrict__ db, int64_t cols, int n,
 // hint_rows_kernel for d = 2^LOGD with the radix-16 register transforms of
 // ntt16.cuh: one block per (prime, DB row), d / 16 threads; a thread reads
 // coefficients tid + (d/16) q of each row block (coalesced), the forward
-// transform leaves it slots 16 tid + q (in [0, 2p), straight into the
+// transform leaves it slots 16 tid + q (unreduced, straight into the
 // Montgomery products with 16-byte loads of V), and the inverse starts from
 // the accumulators. Same residues as hint_rows_kernel. grid = (r, rows),
 // d words of shared memory, needs c.tables16.
@@ -463,7 +457,7 @@ hint_rows16_kernel(const S* __restrict__ db, int64_t cols, int n,
   const int tid = threadIdx.x;
   const uint32_t p = c.p[pi];
   const uint32_t pinv = c.pinv[pi];
-  const uint32_t* tab16 = c.tables16 + static_cast<size_t>(pi) * 4 * d;
+  const uint2* tab16 = c.tables16 + static_cast<size_t>(pi) * 2 * d;
   uint32_t acc[16];
 #pragma unroll
   for (int q = 0; q < 16; ++q) acc[q] = 0;
@@ -472,8 +466,12 @@ hint_rows16_kernel(const S* __restrict__ db, int64_t cols, int n,
     uint32_t x[16];
     const S* rk = src + static_cast<int64_t>(k) * d + tid;  // + NT q: immediates
 #pragma unroll
-    for (int q = 0; q < 16; ++q) x[q] = reduce_u32(static_cast<uint32_t>(rk[NT * q]), p);
-    ntt16_forward<LOGD, false, kCompact, true>(x, smem, tab16, p, tid);
+    for (int q = 0; q < 16; ++q) {
+      // Entries of up to 16 bits are residues as they are.
+      const uint32_t v = static_cast<uint32_t>(rk[NT * q]);
+      x[q] = sizeof(S) <= 2 ? v : reduce_word(v, c, pi);
+    }
+    ntt16_forward<LOGD, false, kCompact>(x, smem, tab16, p, c.one_s[pi], tid);
     const uint4* vk = reinterpret_cast<const uint4*>(
         V + (static_cast<int64_t>(k) * c.r + pi) * d + 16 * tid);
 #pragma unroll
@@ -486,7 +484,7 @@ hint_rows16_kernel(const S* __restrict__ db, int64_t cols, int n,
       }
     }
   }
-  ntt16_inverse<LOGD, false, kCompact>(acc, smem, tab16, p, tid);
+  ntt16_inverse<LOGD, false, kCompact>(acc, smem, tab16 + d, p, c.one_s[pi], tid);
   uint32_t* o = out + (row * c.r + pi) * d + tid;
 #pragma unroll
   for (int q = 0; q < 16; ++q) o[NT * q] = shoup_mul(acc[q], c.scale[pi], c.scale_s[pi], p);
@@ -602,7 +600,7 @@ ext_step_kernel(bool first, const uint32_t* __restrict__ resid_in,
     __syncthreads();
     for (int j = threadIdx.x; j < d; j += blockDim.x) {
       const T dig = gadget_digit<T>(src[j], e.log_q, e.log_digit, e.num_digits, dg);
-      smem[j] = to_residue<T>(dig & static_cast<T>(e.umask), p);
+      smem[j] = reduce_word(static_cast<T>(dig & static_cast<T>(e.umask)), c, pi);
     }
     ntt_forward_t<ITERS>(smem, c, pi);
     const uint32_t* wa =
@@ -676,7 +674,7 @@ ext_step16_kernel(bool first, const uint32_t* __restrict__ resid_in,
   for (int pi = 0; pi < c.r; ++pi) {
     const uint32_t p = c.p[pi];
     const uint32_t pinv = c.pinv[pi];
-    const uint32_t* tab16 = c.tables16 + static_cast<size_t>(pi) * 4 * d;
+    const uint2* tab16 = c.tables16 + static_cast<size_t>(pi) * 2 * d;
     uint32_t acc_a[16], acc_b[16];
 #pragma unroll
     for (int k = 0; k < 16; ++k) acc_a[k] = acc_b[k] = 0;
@@ -689,9 +687,9 @@ ext_step16_kernel(bool first, const uint32_t* __restrict__ resid_in,
       for (int k = 0; k < 16; ++k) {
         const T dig = gadget_digit<T>(src[tid + NT * k], e.log_q, e.log_digit,
                                       e.num_digits, dg);
-        x[k] = to_residue<T>(dig & static_cast<T>(e.umask), p);
+        x[k] = reduce_word(static_cast<T>(dig & static_cast<T>(e.umask)), c, pi);
       }
-      ntt16_forward<LOGD, false, LOGD != 12, true>(x, xs, tab16, p, tid);
+      ntt16_forward<LOGD, false, LOGD != 12>(x, xs, tab16, p, c.one_s[pi], tid);
       const uint4* wa = reinterpret_cast<const uint4*>(
           RGSWa + q * rgswa_qstride + (static_cast<int64_t>(g) * c.r + pi) * d + 16 * tid);
       const uint4* wb = reinterpret_cast<const uint4*>(
@@ -710,12 +708,12 @@ ext_step16_kernel(bool first, const uint32_t* __restrict__ resid_in,
       }
     }
     uint32_t* out = resid_out + rbase + static_cast<int64_t>(pi) * 2 * d;
-    ntt16_inverse<LOGD, false, LOGD != 12>(acc_a, xs, tab16, p, tid);
+    ntt16_inverse<LOGD, false, LOGD != 12>(acc_a, xs, tab16 + d, p, c.one_s[pi], tid);
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
       out[tid + NT * k] = shoup_mul(acc_a[k], c.scale[pi], c.scale_s[pi], p);
     }
-    ntt16_inverse<LOGD, false, LOGD != 12>(acc_b, xs, tab16, p, tid);
+    ntt16_inverse<LOGD, false, LOGD != 12>(acc_b, xs, tab16 + d, p, c.one_s[pi], tid);
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
       out[d + tid + NT * k] = shoup_mul(acc_b[k], c.scale[pi], c.scale_s[pi], p);
@@ -755,7 +753,7 @@ ext_step16_pair_kernel(bool first, const uint32_t* __restrict__ resid_in,
   uint32_t* region = smem + grp * 2 * d;
   T* st = reinterpret_cast<T*>(smem + NGR * 2 * d);  // LowBits of a, then of b
   const int pi = blockIdx.x;
-  const uint32_t* tab16 = c.tables16 + static_cast<size_t>(pi) * 4 * d;
+  const uint2* tab16 = c.tables16 + static_cast<size_t>(pi) * 2 * d;
   const int shard = blockIdx.y;
   const int q = blockIdx.z;
   const int l = gridDim.y;
@@ -787,9 +785,9 @@ ext_step16_pair_kernel(bool first, const uint32_t* __restrict__ resid_in,
     for (int k = 0; k < 16; ++k) {
       const T dig = gadget_digit<T>(src[lt + NT * k], e.log_q, e.log_digit,
                                     e.num_digits, dg);
-      x[k] = to_residue<T>(dig & static_cast<T>(e.umask), p);
+      x[k] = reduce_word(static_cast<T>(dig & static_cast<T>(e.umask)), c, pi);
     }
-    ntt16_forward<LOGD, false, true, true>(x, region, tab16, p, lt, bar);
+    ntt16_forward<LOGD, false, true>(x, region, tab16, p, c.one_s[pi], lt, bar);
     const uint4* wa = reinterpret_cast<const uint4*>(
         RGSWa + q * rgswa_qstride + (static_cast<int64_t>(g) * c.r + pi) * d + 16 * lt);
     const uint4* wb = reinterpret_cast<const uint4*>(
@@ -825,7 +823,7 @@ ext_step16_pair_kernel(bool first, const uint32_t* __restrict__ resid_in,
   }
   __syncthreads();
   if (grp < 2) {
-    ntt16_inverse<LOGD, false, true>(sum, region, tab16, p, lt, bar);
+    ntt16_inverse<LOGD, false, true>(sum, region, tab16 + d, p, c.one_s[pi], lt, bar);
     uint32_t* out = resid_out + rbase + static_cast<int64_t>(pi) * 2 * d + grp * d;
 #pragma unroll
     for (int k = 0; k < 16; ++k) {

@@ -334,8 +334,8 @@ pp_tail_kernel(const T* __restrict__ fin, ChainArgs a, NttCtx c, T* __restrict__
 // the k digit planes of `cur` (k d words of T). The link is a chain of
 // dependent steps, so the digit planes go to shared memory for the
 // transforms (and out to `digits` for the matrix, not read back), and
-// `add` is loaded while other groups finish. Signed digits are below p in
-// magnitude, so their residues need no division. Same words as pp_link.
+// `add` is loaded while other groups finish. Signed digits of up to
+// 27 bits are below p, so their residues need no division. Same words as pp_link.
 template <typename T, int LOGD, int G>
 __device__ __forceinline__ void pp_link16(T* cur, uint32_t* res, uint32_t* xs, T* dig,
                                           const ChainArgs& a, const NttCtx& c, int power,
@@ -359,7 +359,7 @@ __device__ __forceinline__ void pp_link16(T* cur, uint32_t* res, uint32_t* xs, T
   for (int pi = g; pi < c.r; pi += G) {
     const uint32_t p = c.p[pi];
     const uint32_t pinv = c.pinv[pi];
-    const uint32_t* tab16 = c.tables16 + static_cast<size_t>(pi) * 4 * d;
+    const uint2* tab16 = c.tables16 + static_cast<size_t>(pi) * 2 * d;
     uint32_t acc[16];
 #pragma unroll
     for (int q = 0; q < 16; ++q) acc[q] = 0;
@@ -367,12 +367,17 @@ __device__ __forceinline__ void pp_link16(T* cur, uint32_t* res, uint32_t* xs, T
       uint32_t x[16];
 #pragma unroll
       for (int q = 0; q < 16; ++q) {
-        // Digit l of coefficient lt + NT q; |digit| <= 2^(log_digit - 1) < p.
+        // Digit l of coefficient lt + NT q: at most 2^(log_digit - 1) in
+        // magnitude, below p for digits of up to 27 bits.
         const S v = static_cast<S>(dig[l * d + lt + NT * q]);
-        x[q] = v < 0 ? static_cast<uint32_t>(static_cast<int64_t>(v) + p)
-                     : static_cast<uint32_t>(v);
+        if (a.log_digit <= 27) {
+          x[q] = v < 0 ? static_cast<uint32_t>(static_cast<int64_t>(v) + p)
+                       : static_cast<uint32_t>(v);
+        } else {
+          x[q] = pp_signed_residue(static_cast<int64_t>(v), p);
+        }
       }
-      ntt16_forward<LOGD, false, kCompact, true>(x, x_buf, tab16, p, lt, g + 1);
+      ntt16_forward<LOGD, false, kCompact>(x, x_buf, tab16, p, c.one_s[pi], lt, g + 1);
       // Slot 16 lt + q times the key part read through X -> X^power
       // (pp_link's permutation).
       const uint32_t* w = W + (static_cast<int64_t>(l) * c.r + pi) * d;
@@ -385,7 +390,7 @@ __device__ __forceinline__ void pp_link16(T* cur, uint32_t* res, uint32_t* xs, T
         acc[q] = add_mod(acc[q], mont_mul(x[q], __ldg(w + src), p, pinv), p);
       }
     }
-    ntt16_inverse<LOGD, false, kCompact>(acc, x_buf, tab16, p, lt, g + 1);
+    ntt16_inverse<LOGD, false, kCompact>(acc, x_buf, tab16 + d, p, c.one_s[pi], lt, g + 1);
 #pragma unroll
     for (int q = 0; q < 16; ++q) {
       res[static_cast<int64_t>(pi) * d + lt + NT * q] =

@@ -28,6 +28,7 @@
 #include "internal.h"
 #include "limb_gemm.h"
 #include "ntt.cuh"
+#include "answer_poly.cuh"
 #include "poly_kernels.cuh"
 #include "preprocess_kernels.cuh"
 #include "client_kernels.cuh"
@@ -69,9 +70,14 @@ Status Cuda(cudaError_t e, const char* what) {
 // ---------------------------------------------------------------------------
 // Primes and NTT tables.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kPrimes[kMaxPrimes] = {2147352577u, 2146959361u,
-                                          2146041857u, 2145976321u,
-                                          2144796673u};
+// Two sets of primes. 31 bits (c 2^16 + 1): the fewest primes per product, for
+// the transforms of ntt.cuh. 27 bits (c 2^14 + 1): the radix-16 transforms of
+// ntt16.cuh (d = 2048..8192) leave their butterflies unreduced, which needs
+// 32 p < 2^32. Z_2^32 products take three primes of either set.
+enum PrimeSet { kSet31 = 0, kSet27 = 1 };
+constexpr uint32_t kPrimeSets[2][kMaxPrimes] = {
+    {2147352577u, 2146959361u, 2146041857u, 2145976321u, 2144796673u},
+    {133857281u, 133644289u, 133611521u, 133513217u, 133251073u}};
 
 uint64_t PowMod(uint64_t b, uint64_t e, uint64_t m) {
   uint64_t r = 1 % m;
@@ -138,8 +144,8 @@ struct RootPowers {
 // (PowMod per entry, permutation, copy) the tables took 3.2 ms at d = 4096,
 // most of every call that has a ring of its own (client, hint matrix,
 // component entry points). grid = (ceil(d / 256), kMaxPrimes).
-__global__ void ntt_tables_kernel(uint32_t* __restrict__ tables, int logd, bool with16,
-                                  RootPowers rp) {
+__global__ void ntt_tables_kernel(uint32_t* __restrict__ tables, uint2* __restrict__ t16,
+                                  int logd, RootPowers rp) {
   const int d = 1 << logd;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d) return;
@@ -159,14 +165,13 @@ __global__ void ntt_tables_kernel(uint32_t* __restrict__ tables, int logd, bool 
   uint32_t* tab = tables + static_cast<size_t>(pi) * 4 * d;
 #pragma unroll
   for (int part = 0; part < 4; ++part) tab[part * d + i] = v[part];
-  if (!with16) return;
+  if (t16 == nullptr) return;
   // i = m + g' of stage j = log2 i belongs to window w, stage st of it,
   // sub-block x and group g; entry 0 is in no stage and its place in the
   // permuted order (the last one) stays zero.
-  uint32_t* t16 = tables + (static_cast<size_t>(kMaxPrimes) + pi) * 4 * d;
+  uint2* fwd = t16 + static_cast<size_t>(pi) * 2 * d;
   if (i == 0) {
-#pragma unroll
-    for (int part = 0; part < 4; ++part) t16[part * d + d - 1] = 0;
+    fwd[d - 1] = fwd[2 * d - 1] = make_uint2(0, 0);
     return;
   }
   const int stage = 31 - __clz(i);
@@ -180,24 +185,26 @@ __global__ void ntt_tables_kernel(uint32_t* __restrict__ tables, int logd, bool 
   // Ntt16<LOGD>::Base(win) = 15 (1 + 16 + ...) = 16^win - 1.
   const int slot = (1 << (4 * win)) - 1 + (1 << start) * ((1 << st) - (1 << skip)) +
                    x * (1 << start) + g;
-#pragma unroll
-  for (int part = 0; part < 4; ++part) t16[part * d + slot] = v[part];
+  fwd[slot] = make_uint2(v[0], v[1]);
+  fwd[d + slot] = make_uint2(v[2], v[3]);
 }
 
 // Device tables for one ring degree, all primes.
 class NttTables {
  public:
   // The tables are ready for work that follows on `st`.
-  static Status Create(int logd, cudaStream_t st, std::unique_ptr<NttTables>* out) {
+  static Status Create(int logd, PrimeSet set, cudaStream_t st,
+                       std::unique_ptr<NttTables>* out) {
     if (logd < 1 || logd > kLogMaxDegree) {
       return Err(INSPIRE_INVALID_ARGUMENT, "Invalid log_d.");
     }
     std::unique_ptr<NttTables> t(new NttTables());
     t->logd_ = logd;
+    t->set_ = set;
     const int d = 1 << logd;
     RootPowers rp{};
     for (int pi = 0; pi < kMaxPrimes; ++pi) {
-      const uint32_t p = kPrimes[pi];
+      const uint32_t p = kPrimeSets[set][pi];
       uint64_t psi = PowMod(Generator(p), (p - 1) / (2ull * d), p);
       uint64_t psi_inv = PowMod(psi, p - 2, p);
       if (PowMod(psi, d, p) != p - 1) {
@@ -213,11 +220,13 @@ class NttTables {
         psi_inv = psi_inv * psi_inv % p;
       }
     }
-    t->has16_ = logd >= kNtt16MinLogD && logd <= kNtt16MaxLogD;
-    const size_t words = static_cast<size_t>(kMaxPrimes) * 4 * d * (t->has16_ ? 2 : 1);
-    RETURN_IF_ERROR(Cuda(cudaMalloc(&t->dev_, words * 4), "cudaMalloc"));
-    ntt_tables_kernel<<<dim3((d + 255) / 256, kMaxPrimes), 256, 0, st>>>(t->dev_, logd,
-                                                                        t->has16_, rp);
+    const bool has16 = set == kSet27 && logd >= kNtt16MinLogD && logd <= kNtt16MaxLogD;
+    const size_t words = static_cast<size_t>(kMaxPrimes) * 4 * d;
+    RETURN_IF_ERROR(
+        Cuda(cudaMalloc(&t->dev_, words * 4 * (has16 ? 2 : 1)), "cudaMalloc"));
+    if (has16) t->dev16_ = reinterpret_cast<uint2*>(t->dev_ + words);
+    ntt_tables_kernel<<<dim3((d + 255) / 256, kMaxPrimes), 256, 0, st>>>(
+        t->dev_, t->dev16_, logd, rp);
     RETURN_IF_ERROR(Cuda(cudaGetLastError(), "NTT tables"));
     *out = std::move(t);
     return Status{};
@@ -231,8 +240,9 @@ class NttTables {
     c.logd = logd_;
     c.r = r;
     const uint64_t d = 1ull << logd_;
+    const uint32_t* primes = kPrimeSets[set_];
     for (int i = 0; i < kMaxPrimes; ++i) {
-      const uint32_t p = kPrimes[i];
+      const uint32_t p = primes[i];
       c.p[i] = p;
       c.pinv[i] = InvMod2_32(p);
       c.half[i] = (p - 1) / 2;
@@ -240,31 +250,61 @@ class NttTables {
       const uint64_t r32 = (1ull << 32) % p;
       c.scale[i] = static_cast<uint32_t>(dinv * r32 % p);
       c.scale_s[i] = Shoup(c.scale[i], p);
+      c.one_s[i] = Shoup(1, p);
+      c.r32[i] = static_cast<uint32_t>(r32);
+      c.r32_s[i] = Shoup(c.r32[i], p);
       uint64_t prod = 1;
-      for (int j = 0; j < i; ++j) prod *= kPrimes[j];
+      for (int j = 0; j < i; ++j) prod *= primes[j];
       c.pm[i] = prod;
       for (int j = 0; j < kMaxPrimes; ++j) {
-        const uint64_t inv = PowMod(kPrimes[j] % p, p - 2, p);
+        const uint64_t inv = PowMod(primes[j] % p, p - 2, p);
         c.garner[j][i] = j == i ? 0 : static_cast<uint32_t>(inv * r32 % p);
       }
     }
     c.tables = dev_;
-    c.tables16 = has16_ ? dev_ + static_cast<size_t>(kMaxPrimes) * 4 * d : nullptr;
+    c.tables16 = dev16_;
     return c;
+  }
+
+  // Reconstruction constants of r primes (answer_poly.cuh).
+  CrtArgs Crt(int r) const {
+    CrtArgs a{};
+    const uint32_t* primes = kPrimeSets[set_];
+    a.m = 1;
+    for (int i = 0; i < r; ++i) {
+      const uint32_t p = primes[i];
+      uint64_t rest = 1;
+      a.part[i] = 1;
+      for (int j = 0; j < r; ++j) {
+        if (j == i) continue;
+        rest = rest * primes[j] % p;
+        a.part[i] *= primes[j];
+      }
+      const uint64_t dinv = PowMod(1ull << logd_, p - 2, p);
+      a.scale[i] =
+          static_cast<uint32_t>(dinv * ((1ull << 32) % p) % p * PowMod(rest, p - 2, p) % p);
+      a.scale_s[i] = Shoup(a.scale[i], p);
+      a.frac[i] = static_cast<uint32_t>((1ull << 58) / p);
+      a.m *= p;
+    }
+    return a;
   }
 
  private:
   NttTables() = default;
   int logd_ = 0;
-  bool has16_ = false;
+  PrimeSet set_ = kSet31;
   uint32_t* dev_ = nullptr;
+  uint2* dev16_ = nullptr;  // inside dev_'s allocation
 };
 
-// Smallest number of primes whose signed CRT range holds |x| < 2^bits.
-Status PrimesFor(double bits, int* r) {
+// Smallest number of primes of a set whose signed CRT range holds
+// |x| < 2^bits.
+Status PrimesFor(double bits, int* r, PrimeSet set = kSet31) {
+  const uint32_t* primes = kPrimeSets[set];
   for (int n = 1; n <= kMaxPrimes; ++n) {
-    double have = std::log2((kPrimes[n - 1] - 1) / 2.0);
-    for (int j = 0; j < n - 1; ++j) have += std::log2(kPrimes[j]);
+    double have = std::log2((primes[n - 1] - 1) / 2.0);
+    for (int j = 0; j < n - 1; ++j) have += std::log2(primes[j]);
     if (bits < have - 0.01) {
       *r = std::max(n, 2);
       return Status{};
@@ -272,6 +312,15 @@ Status PrimesFor(double bits, int* r) {
   }
   return Err(INSPIRE_INVALID_ARGUMENT,
              "Negacyclic product exceeds the supported exact range.");
+}
+
+// The set for products of up to 2^bits at degree 2^logd: 27-bit primes where
+// the radix-16 transforms run, unless only the larger range holds the product.
+PrimeSet SetFor(int logd, double bits) {
+  int r = 0;
+  return logd >= kNtt16MinLogD && logd <= kNtt16MaxLogD && PrimesFor(bits, &r, kSet27).ok()
+             ? kSet27
+             : kSet31;
 }
 
 // ---------------------------------------------------------------------------
@@ -461,6 +510,8 @@ struct inspire_pir_server {
   inspire::DevBuf db, pack, a_tilde, th_ntt, rgswa_ntt;
   std::unique_ptr<inspire::NttTables> tables;
   inspire::NttCtx ctx_f{}, ctx_e{};
+  bool fused_poly = false;  // answers run answer_poly_kernel
+  inspire::CrtArgs crt{};   // its reconstruction constants
   uint64_t vmask_f = 0, vmask_e = 0, umask_e = 0;
   std::unique_ptr<inspire::LimbGemm> limb;
 
@@ -715,6 +766,60 @@ Status FinalizeStage(inspire_pir_server* s, Workspace* w, int batch,
   return Status{};
 }
 
+// Launches answer_poly_kernel with G groups.
+template <typename T, int LOGD, int G>
+Status LaunchAnswerPoly(const AnswerPolyArgs<T>& a, int l, int batch, cudaStream_t st) {
+  constexpr size_t smem = AnswerPolySmem<T, LOGD, G>();
+  constexpr int R = AnswerPolyPrimes<T>();
+  auto* kernel = answer_poly_kernel<T, LOGD, G, R>;
+  RETURN_IF_ERROR(SetSmem(kernel, smem));
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = R;
+  cluster.val.clusterDim.y = 1;
+  cluster.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(R * l, batch);
+  cfg.blockDim = dim3(G * Ntt16<LOGD>::kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = 1;
+  return Cuda(cudaLaunchKernelEx(&cfg, kernel, a), "polynomial stage");
+}
+
+// The polynomial stage in one launch (answer_poly.cuh). With the 19 x 3 eval
+// gadget there are four live digits over Z_2^32 and six over Z_2^64: a group
+// each where threads and shared memory allow (d = 4096 over Z_2^64: three
+// groups in two rounds).
+template <typename T>
+Status FusedPolyStage(inspire_pir_server* s, Workspace* w, int batch, const T* gemv, T* resp,
+                      cudaStream_t st) {
+  AnswerPolyArgs<T> a;
+  a.th = s->th_ntt.get<uint32_t>();
+  a.yh = w->yh.get<uint32_t>();
+  a.gemv = gemv;
+  a.a_tilde = s->a_tilde.get<T>();
+  a.rgswa = s->rgswa_ntt.get<uint32_t>();
+  a.rgswb = w->rgswb.get<uint32_t>();
+  a.resp = resp;
+  a.k = s->k;
+  a.t = s->t;
+  a.log_q1 = s->prm.log_modulus1_after_switch;
+  a.log_q2 = s->prm.log_modulus2_after_switch;
+  a.e = ExtArgs{s->prm.log_modulus, s->prm.eval_log_digit, s->ne,
+                LiveDigits(s->prm.log_modulus, s->prm.eval_log_digit, s->ne), s->umask_e};
+  a.crt = s->crt;
+  a.c = s->ctx_f;
+  if constexpr (sizeof(T) == 4) {
+    return s->d == 2048 ? LaunchAnswerPoly<T, 11, 4>(a, s->l, batch, st)
+                        : LaunchAnswerPoly<T, 12, 4>(a, s->l, batch, st);
+  } else {
+    return s->d == 2048 ? LaunchAnswerPoly<T, 11, 6>(a, s->l, batch, st)
+                        : LaunchAnswerPoly<T, 12, 3>(a, s->l, batch, st);
+  }
+}
+
 // transforms_done: YhTransform and RgswTransform are already enqueued on a
 // stream that `st` has joined.
 template <typename T>
@@ -723,7 +828,16 @@ Status RunPolyStage(inspire_pir_server* s, Workspace* w, int batch,
                     cudaStream_t st, bool timed, bool transforms_done = false) {
   const int d = s->d, t = s->t, l = s->l, ne = s->ne;
   const int log_q = s->prm.log_modulus;
-  const int nt = PolyThreads(d);
+  if (s->fused_poly) {
+    if (!transforms_done) {
+      RETURN_IF_ERROR(YhTransform<T>(s, w, batch, pkey, st));
+      if (t > 1) RETURN_IF_ERROR(RgswTransform<T>(s, w, batch, sdim, st));
+    }
+    // FinalizeMatrixPack runs inside: its time counts as polynomial
+    // evaluation.
+    if (timed) cudaEventRecord(w->ev[2], st);
+    return FusedPolyStage<T>(s, w, batch, gemv, resp, st);
+  }
   RETURN_IF_ERROR(FinalizeStage<T>(s, w, batch, pkey, gemv, st, transforms_done));
   if (timed) cudaEventRecord(w->ev[2], st);
   const T* a_tilde = s->a_tilde.get<T>();
@@ -1322,24 +1436,40 @@ Status CreateServer(const inspire_pir_params* prm, const void* db,
   if (t > 1 && !se.ok() && s->deferred.ok()) s->deferred = se;
   s->eval_rule = se;
   int r_f = 3, r_e = 3;
+  double bits_f = 0, bits_e = 0;
   if (sf.ok()) {
     s->vmask_f = MaskBits(rf.v_chunks * rf.chunk_bits, cb);
-    RETURN_IF_ERROR(PrimesFor(
-        BoundBits(s->k, d, std::min(rf.u_chunks * rf.chunk_bits, 64),
-                  std::min(rf.v_chunks * rf.chunk_bits, cb)),
-        &r_f));
+    bits_f = BoundBits(s->k, d, std::min(rf.u_chunks * rf.chunk_bits, 64),
+                       std::min(rf.v_chunks * rf.chunk_bits, cb));
   }
   if (se.ok()) {
     s->vmask_e = MaskBits(re.v_chunks * re.chunk_bits, cb);
     s->umask_e = MaskBits(re.u_chunks * re.chunk_bits, cb);
-    RETURN_IF_ERROR(PrimesFor(
-        BoundBits(2 * s->ne, d,
-                  std::min({prm->eval_log_digit, re.u_chunks * re.chunk_bits, cb}),
-                  std::min(re.v_chunks * re.chunk_bits, cb)),
-        &r_e));
+    bits_e = BoundBits(2 * s->ne, d,
+                       std::min({prm->eval_log_digit, re.u_chunks * re.chunk_bits, cb}),
+                       std::min(re.v_chunks * re.chunk_bits, cb));
+  }
+  const PrimeSet set = SetFor(prm->log_degree, std::max(bits_f, bits_e));
+  if (sf.ok()) RETURN_IF_ERROR(PrimesFor(bits_f, &r_f, set));
+  if (se.ok()) RETURN_IF_ERROR(PrimesFor(bits_e, &r_e, set));
+  // The fused polynomial stage adds a slice's two products before the inverse
+  // transform: one prime count for both, holding their sum (a bit more than
+  // the larger). d = 8192 has no room for its tables and regions in shared
+  // memory.
+  if (set == kSet27 && d <= 4096 && sf.ok() && (t == 1 || se.ok())) {
+    int need = 0;
+    const int r = cb == 32 ? AnswerPolyPrimes<uint32_t>() : AnswerPolyPrimes<uint64_t>();
+    const double bits = t == 1 ? bits_f : std::max(bits_f, bits_e) + 1;
+    // Its 64-bit sums of products below 2^59 take 30 terms.
+    const int terms =
+        s->k + (t > 1 ? 2 * LiveDigits(prm->log_modulus, prm->eval_log_digit, s->ne) : 0);
+    if (PrimesFor(bits, &need, set).ok() && need <= r && terms <= 30) {
+      s->fused_poly = true;
+      r_f = r_e = r;
+    }
   }
   // The server's calls come on streams of their own: wait for the tables.
-  RETURN_IF_ERROR(NttTables::Create(prm->log_degree, nullptr, &s->tables));
+  RETURN_IF_ERROR(NttTables::Create(prm->log_degree, set, nullptr, &s->tables));
   RETURN_IF_ERROR(Cuda(cudaStreamSynchronize(nullptr), "NTT tables"));
   {
     int dev = 0;
@@ -1348,6 +1478,7 @@ Status CreateServer(const inspire_pir_params* prm, const void* db,
     }
   }
   s->ctx_f = s->tables->Ctx(r_f);
+  if (s->fused_poly) s->crt = s->tables->Crt(r_f);
   s->ctx_e = s->tables->Ctx(r_e);
 
   const size_t w = Words(cb);
@@ -3171,7 +3302,7 @@ int inspire_inner_product(int32_t coeff_bits, const void* u, const void* v,
   st = PrimesFor(BoundBits(n, d, ub, vb), &r);
   if (!st.ok()) return Report(st, err, err_len);
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, nullptr, &tabs);
+  st = NttTables::Create(logd, kSet31, nullptr, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   NttCtx c = tabs->Ctx(r);
   const size_t total = static_cast<size_t>(n) * d;
@@ -3268,11 +3399,13 @@ int inspire_compute_hint_matrix(int32_t db_kind, int32_t coeff_bits, const void*
   }
   const int s_bits = 8 * elem_size(db_kind);
   int r = 0;
-  Status st = PrimesFor(BoundBits(n, d, s_bits, coeff_bits), &r);
+  const double bits = BoundBits(n, d, s_bits, coeff_bits);
+  const PrimeSet set = SetFor(logd, bits);
+  Status st = PrimesFor(bits, &r, set);
   if (!st.ok()) return Report(st, err, err_len);
   const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, cs, &tabs);
+  st = NttTables::Create(logd, set, cs, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   NttCtx c = tabs->Ctx(r);
   int dev = 0, sms = 152;
@@ -3401,7 +3534,7 @@ int inspire_external_product(const inspire_pir_params* params,
                  &r);
   if (!st.ok()) return Report(st, err, err_len);
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(params->log_degree, nullptr, &tabs);
+  st = NttTables::Create(params->log_degree, kSet31, nullptr, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   NttCtx c = tabs->Ctx(r);
   const size_t w = cb / 8;
@@ -3493,7 +3626,9 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
   }
   const int k = num_digits;
   int r = 0;
-  Status st = PrimesFor(BoundBits(k, d, log_digit, coeff_bits), &r);
+  const double bits = BoundBits(k, d, log_digit, coeff_bits);
+  const PrimeSet set = SetFor(logd, bits);
+  Status st = PrimesFor(bits, &r, set);
   if (!st.ok()) return Report(st, err, err_len);
   const int iters = d > 4096 ? 2 : 1;
   const int threads = d / (4 * iters);
@@ -3502,7 +3637,7 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
   if (chain_smem > 227 * 1024) return fail("ring degree and gadget too large.");
   const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, cs, &tabs);
+  st = NttTables::Create(logd, set, cs, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   const NttCtx c = tabs->Ctx(r);
   const size_t mw = elem_size(mat_kind);
@@ -3730,7 +3865,7 @@ int inspire_client_create_requests(const inspire_pir_params* params,
   if (!st.ok()) return Report(st, err, err_len);
   const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, cs, &tabs);
+  st = NttTables::Create(logd, kSet31, cs, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   const NttCtx c = tabs->Ctx(r);
   const size_t w = cb / 8;
@@ -3822,7 +3957,7 @@ int inspire_client_process_responses(const inspire_pir_params* params,
   if (!st.ok()) return Report(st, err, err_len);
   const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, cs, &tabs);
+  st = NttTables::Create(logd, kSet31, cs, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   const NttCtx c = tabs->Ctx(r);
   const size_t w = cb / 8;
@@ -3892,7 +4027,7 @@ int inspire_finalize_matrix_pack(const inspire_pir_params* params,
                  &r);
   if (!st.ok()) return Report(st, err, err_len);
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(params->log_degree, nullptr, &tabs);
+  st = NttTables::Create(params->log_degree, kSet31, nullptr, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   NttCtx c = tabs->Ctx(r);
   const size_t w = cb / 8;
