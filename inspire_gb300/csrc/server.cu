@@ -29,6 +29,7 @@
 #include "limb_gemm.h"
 #include "ntt.cuh"
 #include "answer_poly.cuh"
+#include "hint16.cuh"
 #include "poly_kernels.cuh"
 #include "preprocess_kernels.cuh"
 #include "client_kernels.cuh"
@@ -3399,9 +3400,11 @@ int inspire_compute_hint_matrix(int32_t db_kind, int32_t coeff_bits, const void*
   }
   const int s_bits = 8 * elem_size(db_kind);
   int r = 0;
-  const double bits = BoundBits(n, d, s_bits, coeff_bits);
-  const PrimeSet set = SetFor(logd, bits);
-  Status st = PrimesFor(bits, &r, set);
+  // d = 2048..8192: 27-bit primes, the a-components in halves (hint16.cuh).
+  const bool halves = logd >= kNtt16MinLogD && logd <= kNtt16MaxLogD;
+  const PrimeSet set = halves ? kSet27 : kSet31;
+  Status st = PrimesFor(
+      BoundBits(n, d, s_bits, halves ? coeff_bits / kHintParts : coeff_bits), &r, set);
   if (!st.ok()) return Report(st, err, err_len);
   const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   std::unique_ptr<NttTables> tabs;
@@ -3414,71 +3417,55 @@ int inspire_compute_hint_matrix(int32_t db_kind, int32_t coeff_bits, const void*
   }
   const size_t w = coeff_bits / 8;
   const size_t es = elem_size(db_kind);
-  // The a-components on the host (a device copy comes back first: they are
-  // n * d words).
-  std::vector<uint8_t> a_host(static_cast<size_t>(n) * d * w);
-  if (on_device) {
-    st = Cuda(cudaMemcpy(a_host.data(), a_components, a_host.size(), cudaMemcpyDeviceToHost),
-              "a-components download");
-    if (!st.ok()) return Report(st, err, err_len);
-  } else {
-    std::memcpy(a_host.data(), a_components, a_host.size());
-  }
-  // v_k[0] = a_k[0], v_k[j] = -a_k[d - j] (hint_computation.cc:110-119).
-  std::vector<uint8_t> vinv(static_cast<size_t>(n) * d * w);
-  for (int k = 0; k < n; ++k) {
-    for (int j = 0; j < d; ++j) {
-      const int src = j == 0 ? 0 : d - j;
-      const uint8_t* a = a_host.data() + (static_cast<size_t>(k) * d + src) * w;
-      uint8_t* v = vinv.data() + (static_cast<size_t>(k) * d + j) * w;
-      if (w == 4) {
-        uint32_t x;
-        std::memcpy(&x, a, 4);
-        x = j == 0 ? x : 0u - x;
-        std::memcpy(v, &x, 4);
-      } else {
-        uint64_t x;
-        std::memcpy(&x, a, 8);
-        x = j == 0 ? x : 0ull - x;
-        std::memcpy(v, &x, 8);
-      }
-    }
-  }
-  DevBuf dv, dV, dres, ddb, dout;
-  st = dv.Upload(vinv.data(), vinv.size());
-  if (st.ok()) st = dV.Alloc(static_cast<size_t>(n) * r * d * 4);
-  if (st.ok()) st = dres.Alloc(static_cast<size_t>(rows) * r * d * 4);
+  DevBuf da, dV, dres, ddb, dout;
+  const void* a_dev = a_components;
   const void* db_dev = db;
   void* out_dev = out;
-  if (st.ok() && !on_device) {
-    st = ddb.Upload(db, static_cast<size_t>(rows) * cols * es);
+  const size_t a_words = static_cast<size_t>(n) * d;
+  if (!on_device) {
+    st = da.Upload(a_components, a_words * w);
+    if (st.ok()) st = ddb.Upload(db, static_cast<size_t>(rows) * cols * es);
     if (st.ok()) st = dout.Alloc(static_cast<size_t>(rows) * d * w);
+    a_dev = da.get();
     db_dev = ddb.get();
     out_dev = dout.get();
+  }
+  if (st.ok()) st = dV.Alloc(a_words * r * 4 * (halves ? kHintParts : 1));
+  if (st.ok() && !halves) {
+    // [rows][r][d] residues, and the inverted a-components before that.
+    st = dres.Alloc(std::max(static_cast<size_t>(rows) * r * d * 4, a_words * w));
   }
   if (st.ok()) {
     auto run = [&](auto ttag, auto stag) -> Status {
       using T = decltype(ttag);
       using S = decltype(stag);
-      ntt_coeffs_kernel<T><<<dim3(n * r, 1), PolyThreads(d), d * 4, cs>>>(
-          dv.get<T>(), 0, 0, n, static_cast<T>(~0ull), dV.get<uint32_t>(), d, c);
-      RETURN_IF_ERROR(Cuda(cudaGetLastError(), "a-component transforms"));
-      const dim3 grid(r, static_cast<unsigned>(rows));
-      if (c.tables16 != nullptr) {
-        // d = 2048..8192: the radix-16 register transforms.
+      const T* a = static_cast<const T*>(a_dev);
+      if (halves) {
+        const CrtArgs crt = tabs->Crt(r);
         INSPIRE_NTT16_DISPATCH(
-            c.logd, RETURN_IF_ERROR(SetSmem(hint_rows16_kernel<S, LG>, d * 4));
-            hint_rows16_kernel<S, LG><<<grid, Ntt16<LG>::kThreads, d * 4, cs>>>(
+            c.logd,
+            hint_parts16_kernel<T, LG><<<dim3(kHintParts * n, r), Ntt16<LG>::kThreads, 0, cs>>>(
+                a, dV.get<uint32_t>(), c);
+            RETURN_IF_ERROR(Cuda(cudaGetLastError(), "a-component transforms"));
+            const size_t smem = HintRowsSmem<T, LG>();
+            RETURN_IF_ERROR(SetSmem(hint_rows16_kernel<T, S, LG>, smem));
+            hint_rows16_kernel<T, S, LG>
+            <<<static_cast<unsigned>(rows), Ntt16<LG>::kThreads, smem, cs>>>(
                 static_cast<const S*>(db_dev), cols, n, dV.get<uint32_t>(),
-                dres.get<uint32_t>(), c));
-      } else {
-        const PolyLaunch pl = PolyShapeFor(d, static_cast<int64_t>(r) * rows, sms);
-        INSPIRE_ITERS_DISPATCH(
-            pl.iters, RETURN_IF_ERROR(SetSmem(hint_rows_kernel<S, IT>, d * 4));
-            hint_rows_kernel<S, IT><<<grid, pl.nt, d * 4, cs>>>(
-                static_cast<const S*>(db_dev), cols, n, dV.get<uint32_t>(),
-                dres.get<uint32_t>(), c));
+                static_cast<T*>(out_dev), c, crt));
+        return Cuda(cudaGetLastError(), "hint rows");
       }
+      invert_components_kernel<T><<<dim3((d + 255) / 256, n), 256, 0, cs>>>(a, d, dres.get<T>());
+      RETURN_IF_ERROR(Cuda(cudaGetLastError(), "a-component inversion"));
+      ntt_coeffs_kernel<T><<<dim3(n * r, 1), PolyThreads(d), d * 4, cs>>>(
+          dres.get<T>(), 0, 0, n, static_cast<T>(~0ull), dV.get<uint32_t>(), d, c);
+      RETURN_IF_ERROR(Cuda(cudaGetLastError(), "a-component transforms"));
+      const PolyLaunch pl = PolyShapeFor(d, static_cast<int64_t>(r) * rows, sms);
+      INSPIRE_ITERS_DISPATCH(
+          pl.iters, RETURN_IF_ERROR(SetSmem(hint_rows_kernel<S, IT>, d * 4));
+          hint_rows_kernel<S, IT><<<dim3(r, static_cast<unsigned>(rows)), pl.nt, d * 4, cs>>>(
+              static_cast<const S*>(db_dev), cols, n, dV.get<uint32_t>(),
+              dres.get<uint32_t>(), c));
       RETURN_IF_ERROR(Cuda(cudaGetLastError(), "hint rows"));
       const int64_t total = rows * static_cast<int64_t>(d);
       const unsigned blocks = static_cast<unsigned>(std::min<int64_t>((total + 255) / 256, 152 * 8));
