@@ -129,6 +129,128 @@ int BitRev(int x, int bits) {
   return r;
 }
 
+// Small temporaries of the calls that keep no state (client, hint matrix,
+// PreprocessMatrixPack: twiddle tables and transforms) come from a memory pool
+// of the device, in stream order: a cudaMalloc and cudaFree pair took 75 us of
+// such a call, a pool allocation 10. At most kScratchPoolBytes stay with the
+// pool when idle (its release threshold; what exceeds it goes back at the
+// next synchronisation), and all of it when an allocation fails for lack of
+// memory. The CUDA pool serialises threads and orders reuse between streams.
+constexpr size_t kScratchPoolBytes = 32u << 20;
+constexpr int kScratchDevices = 64;
+
+// The current device's pool; null if it has none (callers then use cudaMalloc).
+cudaMemPool_t ScratchPool() {
+  static std::mutex mu;
+  static cudaMemPool_t pools[kScratchDevices] = {};
+  static bool tried[kScratchDevices] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kScratchDevices) return nullptr;
+  std::lock_guard<std::mutex> lock(mu);
+  if (!tried[dev]) {
+    tried[dev] = true;
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    uint64_t keep = kScratchPoolBytes;
+    if (cudaMemPoolCreate(&pool, &props) == cudaSuccess) {
+      if (cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess) {
+        pools[dev] = pool;
+      } else {
+        cudaMemPoolDestroy(pool);
+      }
+    }
+    cudaGetLastError();
+  }
+  return pools[dev];
+}
+
+// ---------------------------------------------------------------------------
+// RAII device buffer.
+// ---------------------------------------------------------------------------
+class DevBuf {
+ public:
+  DevBuf() = default;
+  ~DevBuf() { Free(); }
+  DevBuf(const DevBuf&) = delete;
+  DevBuf& operator=(const DevBuf&) = delete;
+  Status Alloc(size_t bytes) {
+    Free();
+    if (bytes == 0) return Status{};
+    cudaError_t e = cudaMalloc(&ptr_, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+      // The pool's idle memory goes back before the allocation fails.
+      cudaGetLastError();
+      if (cudaMemPool_t pool = ScratchPool()) cudaMemPoolTrimTo(pool, 0);
+      e = cudaMalloc(&ptr_, bytes);
+    }
+    if (e != cudaSuccess) {
+      ptr_ = nullptr;
+      return Err(INSPIRE_RESOURCE_EXHAUSTED,
+                 std::string("GPU allocation of ") + std::to_string(bytes) +
+                     " bytes failed: " + cudaGetErrorString(e));
+    }
+    bytes_ = bytes;
+    return Status{};
+  }
+  // A temporary of a call whose work runs on `st`: from the scratch pool when
+  // it is small, else as Alloc.
+  Status AllocScratch(size_t bytes, cudaStream_t st) {
+    cudaMemPool_t pool = bytes > 0 && bytes <= kScratchPoolBytes ? ScratchPool() : nullptr;
+    if (pool == nullptr) return Alloc(bytes);
+    Free();
+    if (cudaMallocFromPoolAsync(&ptr_, bytes, pool, st) != cudaSuccess) {
+      ptr_ = nullptr;
+      cudaGetLastError();
+      return Alloc(bytes);
+    }
+    pooled_ = true;
+    stream_ = st;
+    bytes_ = bytes;
+    return Status{};
+  }
+  Status Upload(const void* host, size_t bytes) {
+    RETURN_IF_ERROR(Alloc(bytes));
+    if (bytes == 0) return Status{};
+    return Cuda(cudaMemcpy(ptr_, host, bytes, cudaMemcpyHostToDevice),
+                "cudaMemcpy H2D");
+  }
+  void Free() {
+    if (ptr_ && pooled_) {
+      cudaFreeAsync(ptr_, stream_);
+    } else if (ptr_) {
+      cudaFree(ptr_);
+    }
+    ptr_ = nullptr;
+    bytes_ = 0;
+    pooled_ = false;
+  }
+  // Moves another buffer's allocation into this one.
+  void Take(DevBuf* other) {
+    Free();
+    ptr_ = other->ptr_;
+    bytes_ = other->bytes_;
+    pooled_ = other->pooled_;
+    stream_ = other->stream_;
+    other->ptr_ = nullptr;
+    other->bytes_ = 0;
+    other->pooled_ = false;
+  }
+  template <typename P = void>
+  P* get() const {
+    return static_cast<P*>(ptr_);
+  }
+  size_t bytes() const { return bytes_; }
+
+ private:
+  void* ptr_ = nullptr;
+  size_t bytes_ = 0;
+  bool pooled_ = false;
+  cudaStream_t stream_ = nullptr;
+};
+
 // psi^(2^j) and psi^-(2^j) mod p (j < log d) with their Shoup constants: what
 // ntt_tables_kernel multiplies up into every twiddle.
 struct RootPowers {
@@ -193,9 +315,10 @@ __global__ void ntt_tables_kernel(uint32_t* __restrict__ tables, uint2* __restri
 // Device tables for one ring degree, all primes.
 class NttTables {
  public:
-  // The tables are ready for work that follows on `st`.
+  // The tables are ready for work that follows on `st`. scratch: they are a
+  // temporary of one call.
   static Status Create(int logd, PrimeSet set, cudaStream_t st,
-                       std::unique_ptr<NttTables>* out) {
+                       std::unique_ptr<NttTables>* out, bool scratch = true) {
     if (logd < 1 || logd > kLogMaxDegree) {
       return Err(INSPIRE_INVALID_ARGUMENT, "Invalid log_d.");
     }
@@ -223,17 +346,14 @@ class NttTables {
     }
     const bool has16 = set == kSet27 && logd >= kNtt16MinLogD && logd <= kNtt16MaxLogD;
     const size_t words = static_cast<size_t>(kMaxPrimes) * 4 * d;
-    RETURN_IF_ERROR(
-        Cuda(cudaMalloc(&t->dev_, words * 4 * (has16 ? 2 : 1)), "cudaMalloc"));
-    if (has16) t->dev16_ = reinterpret_cast<uint2*>(t->dev_ + words);
+    const size_t bytes = words * 4 * (has16 ? 2 : 1);
+    RETURN_IF_ERROR(scratch ? t->mem_.AllocScratch(bytes, st) : t->mem_.Alloc(bytes));
+    if (has16) t->dev16_ = reinterpret_cast<uint2*>(t->mem_.get<uint32_t>() + words);
     ntt_tables_kernel<<<dim3((d + 255) / 256, kMaxPrimes), 256, 0, st>>>(
-        t->dev_, t->dev16_, logd, rp);
+        t->mem_.get<uint32_t>(), t->dev16_, logd, rp);
     RETURN_IF_ERROR(Cuda(cudaGetLastError(), "NTT tables"));
     *out = std::move(t);
     return Status{};
-  }
-  ~NttTables() {
-    if (dev_) cudaFree(dev_);
   }
 
   NttCtx Ctx(int r) const {
@@ -262,7 +382,7 @@ class NttTables {
         c.garner[j][i] = j == i ? 0 : static_cast<uint32_t>(inv * r32 % p);
       }
     }
-    c.tables = dev_;
+    c.tables = mem_.get<uint32_t>();
     c.tables16 = dev16_;
     return c;
   }
@@ -295,8 +415,8 @@ class NttTables {
   NttTables() = default;
   int logd_ = 0;
   PrimeSet set_ = kSet31;
-  uint32_t* dev_ = nullptr;
-  uint2* dev16_ = nullptr;  // inside dev_'s allocation
+  DevBuf mem_;
+  uint2* dev16_ = nullptr;  // inside mem_
 };
 
 // Smallest number of primes of a set whose signed CRT range holds
@@ -385,58 +505,6 @@ double BoundBits(int n, int d, double u_bits, double v_bits) {
 }
 
 size_t Words(int coeff_bits) { return coeff_bits / 8; }
-
-// ---------------------------------------------------------------------------
-// RAII device buffer.
-// ---------------------------------------------------------------------------
-class DevBuf {
- public:
-  DevBuf() = default;
-  ~DevBuf() { Free(); }
-  DevBuf(const DevBuf&) = delete;
-  DevBuf& operator=(const DevBuf&) = delete;
-  Status Alloc(size_t bytes) {
-    Free();
-    if (bytes == 0) return Status{};
-    cudaError_t e = cudaMalloc(&ptr_, bytes);
-    if (e != cudaSuccess) {
-      ptr_ = nullptr;
-      return Err(INSPIRE_RESOURCE_EXHAUSTED,
-                 std::string("GPU allocation of ") + std::to_string(bytes) +
-                     " bytes failed: " + cudaGetErrorString(e));
-    }
-    bytes_ = bytes;
-    return Status{};
-  }
-  Status Upload(const void* host, size_t bytes) {
-    RETURN_IF_ERROR(Alloc(bytes));
-    if (bytes == 0) return Status{};
-    return Cuda(cudaMemcpy(ptr_, host, bytes, cudaMemcpyHostToDevice),
-                "cudaMemcpy H2D");
-  }
-  void Free() {
-    if (ptr_) cudaFree(ptr_);
-    ptr_ = nullptr;
-    bytes_ = 0;
-  }
-  // Moves another buffer's allocation into this one.
-  void Take(DevBuf* other) {
-    Free();
-    ptr_ = other->ptr_;
-    bytes_ = other->bytes_;
-    other->ptr_ = nullptr;
-    other->bytes_ = 0;
-  }
-  template <typename P = void>
-  P* get() const {
-    return static_cast<P*>(ptr_);
-  }
-  size_t bytes() const { return bytes_; }
-
- private:
-  void* ptr_ = nullptr;
-  size_t bytes_ = 0;
-};
 
 template <typename K>
 Status SetSmem(K kernel, size_t bytes) {
@@ -1470,7 +1538,7 @@ Status CreateServer(const inspire_pir_params* prm, const void* db,
     }
   }
   // The server's calls come on streams of their own: wait for the tables.
-  RETURN_IF_ERROR(NttTables::Create(prm->log_degree, set, nullptr, &s->tables));
+  RETURN_IF_ERROR(NttTables::Create(prm->log_degree, set, nullptr, &s->tables, false));
   RETURN_IF_ERROR(Cuda(cudaStreamSynchronize(nullptr), "NTT tables"));
   {
     int dev = 0;
@@ -3430,7 +3498,7 @@ int inspire_compute_hint_matrix(int32_t db_kind, int32_t coeff_bits, const void*
     db_dev = ddb.get();
     out_dev = dout.get();
   }
-  if (st.ok()) st = dV.Alloc(a_words * r * 4 * (halves ? kHintParts : 1));
+  if (st.ok()) st = dV.AllocScratch(a_words * r * 4 * (halves ? kHintParts : 1), cs);
   if (st.ok() && !halves) {
     // [rows][r][d] residues, and the inverted a-components before that.
     st = dres.Alloc(std::max(static_cast<size_t>(rows) * r * d * 4, a_words * w));
@@ -3848,11 +3916,13 @@ int inspire_client_create_requests(const inspire_pir_params* params,
     }
   }
   int r = 0;
-  Status st = PrimesFor(BoundBits(1, d, cb, 2), &r);
+  const double bits = BoundBits(1, d, cb, 2);
+  const PrimeSet set = SetFor(logd, bits);
+  Status st = PrimesFor(bits, &r, set);
   if (!st.ok()) return Report(st, err, err_len);
   const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, kSet31, cs, &tabs);
+  st = NttTables::Create(logd, set, cs, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   const NttCtx c = tabs->Ctx(r);
   const size_t w = cb / 8;
@@ -3875,7 +3945,11 @@ int inspire_client_create_requests(const inspire_pir_params* params,
     sd_out = dsd.get();
     pk_out = dpk.get();
   }
-  if (st.ok()) st = dshat.Alloc(static_cast<size_t>(batch) * r * d * 4);
+  // The keys' transforms, then the a-components' (radix-16 rings).
+  const size_t hat_words = static_cast<size_t>(r) * d;
+  if (st.ok()) {
+    st = dshat.AllocScratch((batch + (set == kSet27 ? rows : 0)) * hat_words * 4, cs);
+  }
   ClientArgs ca;
   ca.d = d;
   ca.log_d = logd;
@@ -3897,6 +3971,22 @@ int inspire_client_create_requests(const inspire_pir_params* params,
   const size_t smem = static_cast<size_t>(r) * d * 4;
   auto run = [&](auto tag) -> Status {
     using T = decltype(tag);
+    if (set == kSet27) {
+      const CrtArgs crt = tabs->Crt(r);
+      uint32_t* s_hat = dshat.get<uint32_t>();
+      uint32_t* a_hat = s_hat + batch * hat_words;
+      INSPIRE_NTT16_DISPATCH(
+          logd,
+          cl_transforms16_kernel<T, LG>
+          <<<dim3(static_cast<unsigned>(rows + batch), r), Ntt16<LG>::kThreads, 0, cs>>>(
+              static_cast<const T*>(a_dev), keys, static_cast<int>(rows), a_hat, s_hat, c);
+          RETURN_IF_ERROR(SetSmem(cl_request16_kernel<T, LG>, d * sizeof(T)));
+          cl_request16_kernel<T, LG>
+          <<<dim3(static_cast<unsigned>(rows), batch), Ntt16<LG>::kThreads, d * sizeof(T), cs>>>(
+              a_hat, s_hat, ca, c, crt, static_cast<T*>(fd_out), static_cast<T*>(sd_out),
+              static_cast<T*>(pk_out)));
+      return Cuda(cudaGetLastError(), "client requests");
+    }
     auto go = [&](auto itag) -> Status {
       constexpr int IT = decltype(itag)::value;
       RETURN_IF_ERROR(SetSmem(cl_key_ntt_kernel<IT>, d * 4));
@@ -3940,11 +4030,13 @@ int inspire_client_process_responses(const inspire_pir_params* params,
   const int l = params->entry_size_multiple;
   if (l <= 0) return fail("entry_size_multiple must be positive.");
   int r = 0;
-  Status st = PrimesFor(BoundBits(1, d, cb, 2), &r);
+  const double bits = BoundBits(1, d, cb, 2);
+  const PrimeSet set = SetFor(logd, bits);
+  Status st = PrimesFor(bits, &r, set);
   if (!st.ok()) return Report(st, err, err_len);
   const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
   std::unique_ptr<NttTables> tabs;
-  st = NttTables::Create(logd, kSet31, cs, &tabs);
+  st = NttTables::Create(logd, set, cs, &tabs);
   if (!st.ok()) return Report(st, err, err_len);
   const NttCtx c = tabs->Ctx(r);
   const size_t w = cb / 8;
@@ -3960,12 +4052,27 @@ int inspire_client_process_responses(const inspire_pir_params* params,
     resp = dresp.get();
     o = dout.get();
   }
-  if (st.ok()) st = dshat.Alloc(static_cast<size_t>(batch) * r * d * 4);
+  if (st.ok() && set != kSet27) {
+    st = dshat.AllocScratch(static_cast<size_t>(batch) * r * d * 4, cs);
+  }
   const int iters = d > 4096 ? 2 : 1;
   const int threads = d / (4 * iters);
   const size_t smem = static_cast<size_t>(r) * d * 4;
   auto run = [&](auto tag) -> Status {
     using T = decltype(tag);
+    if (set == kSet27) {
+      const CrtArgs crt = tabs->Crt(r);
+      INSPIRE_NTT16_DISPATCH(
+          logd, constexpr int G = LG <= 12 ? 2 : 1;
+          const size_t smem16 = static_cast<size_t>(r + G) * d * 4;
+          RETURN_IF_ERROR(SetSmem(cl_decrypt16_kernel<T, LG, G>, smem16));
+          cl_decrypt16_kernel<T, LG, G>
+          <<<dim3(l, batch), G * Ntt16<LG>::kThreads, smem16, cs>>>(
+              static_cast<const T*>(resp), keys, l, params->log_modulus1_after_switch,
+              params->log_modulus2_after_switch, params->plaintext_modulus, c, crt,
+              static_cast<T*>(o)));
+      return Cuda(cudaGetLastError(), "client decryption");
+    }
     auto go = [&](auto itag) -> Status {
       constexpr int IT = decltype(itag)::value;
       RETURN_IF_ERROR(SetSmem(cl_key_ntt_kernel<IT>, d * 4));
