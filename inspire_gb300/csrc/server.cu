@@ -33,6 +33,7 @@
 #include "poly_kernels.cuh"
 #include "preprocess_kernels.cuh"
 #include "client_kernels.cuh"
+#include "chain16.cuh"
 #include "server_api.h"
 
 namespace inspire {
@@ -3685,6 +3686,14 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
   const PrimeSet set = SetFor(logd, bits);
   Status st = PrimesFor(bits, &r, set);
   if (!st.ok()) return Report(st, err, err_len);
+  // d = 2048 and 4096: a cluster per chain (chain16.cuh), with as many primes
+  // as its code is built for.
+  const int chain_r = coeff_bits == 32 ? AnswerPolyPrimes<uint32_t>() : AnswerPolyPrimes<uint64_t>();
+  const size_t cluster_smem =
+      logd == 11 ? Chain16Smem<11>(k) : logd == 12 ? Chain16Smem<12>(k) : SIZE_MAX;
+  const bool clusters = set == kSet27 && r <= chain_r && log_digit <= 27 && k <= 30 &&
+                        cluster_smem <= 227 * 1024;
+  if (clusters) r = chain_r;
   const int iters = d > 4096 ? 2 : 1;
   const int threads = d / (4 * iters);
   const size_t w = coeff_bits / 8;
@@ -3817,6 +3826,35 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
           dfin.get<T>(), ca, c, static_cast<T*>(th_out), static_cast<T*>(a_out));
       return Cuda(cudaGetLastError(), "a_tilde_agg");
     };
+    auto chain_clusters = [&](auto ltag) -> Status {
+      constexpr int LG = decltype(ltag)::value;
+      constexpr int GR = 4;
+      constexpr int R = AnswerPolyPrimes<T>();
+      auto* kernel = chain16_cluster_kernel<T, LG, GR, R>;
+      RETURN_IF_ERROR(SetSmem(kernel, cluster_smem));
+      cudaLaunchAttribute cluster;
+      cluster.id = cudaLaunchAttributeClusterDimension;
+      cluster.val.clusterDim.x = R;
+      cluster.val.clusterDim.y = 1;
+      cluster.val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(2 * R, slices);
+      cfg.blockDim = dim3(GR * Ntt16<LG>::kThreads);
+      cfg.dynamicSmemBytes = cluster_smem;
+      cfg.stream = cs;
+      cfg.attrs = &cluster;
+      cfg.numAttrs = 1;
+      const CrtArgs crt = tabs->Crt(R);
+      RETURN_IF_ERROR(Cuda(cudaLaunchKernelEx(&cfg, kernel, ev->get<T>(), ca, c, crt,
+                                              dtg.get<T>(), dtgh.get<T>(), dfin.get<T>()),
+                           "reduction chains"));
+      constexpr int GT = LG == 11 ? 3 : 2;
+      const size_t smem16 = (1 + k) * d * w + static_cast<size_t>(d) * 4 * (r + GT);
+      RETURN_IF_ERROR(SetSmem(pp_tail16_kernel<T, LG, GT>, smem16));
+      pp_tail16_kernel<T, LG, GT><<<slices, GT * Ntt16<LG>::kThreads, smem16, cs>>>(
+          dfin.get<T>(), ca, c, static_cast<T*>(th_out), static_cast<T*>(a_out));
+      return Cuda(cudaGetLastError(), "a_tilde_agg");
+    };
     using I1 = std::integral_constant<int, 1>;
     using I2 = std::integral_constant<int, 2>;
     using I3 = std::integral_constant<int, 3>;
@@ -3825,7 +3863,13 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
     const int groups16 = logd == 11 ? std::min(r, 5) : logd == 12 ? std::min(r, 3) : 1;
     const bool fits16 =
         (1 + k) * d * w + static_cast<size_t>(d) * 4 * (r + groups16) <= 227 * 1024;
-    if (c.tables16 != nullptr && fits16 && logd == 11) {
+    if (clusters && fits16) {
+      if (logd == 11) {
+        RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 11>{}));
+      } else {
+        RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 12>{}));
+      }
+    } else if (c.tables16 != nullptr && fits16 && logd == 11) {
       if (groups16 == 2) RETURN_IF_ERROR(chains16(std::integral_constant<int, 11>{}, I2{}));
       if (groups16 == 3) RETURN_IF_ERROR(chains16(std::integral_constant<int, 11>{}, I3{}));
       if (groups16 == 4) RETURN_IF_ERROR(chains16(std::integral_constant<int, 11>{}, I4{}));
