@@ -9,7 +9,7 @@
 //    coefficients are ring elements (a_hat_agg and the matrix blocks): a
 //    radix-2 decimation-in-frequency transform whose twiddles are monomials,
 //    so every butterfly is an add, a subtract and a signed rotation of whole
-//    polynomials, one stage per launch over all (pair, coefficient) cells;
+//    polynomials, up to three stages per pass over memory;
 //  * the reduction chains of PreprocessPack: a sequential run of d/2 - 1
 //    gadget decompositions and inner products with automorphed key parts,
 //    one block per chain, the products as exact multi-prime NTTs in shared
@@ -68,58 +68,105 @@ __global__ void pp_atilde_kernel(const T* __restrict__ hint, int64_t stride, int
   }
 }
 
-// One radix-2 decimation-in-frequency stage of E[m] = sum_i c[i] X^{2im}
-// (d polynomials of length d per slice; natural order in, bit-reversed order
-// out once all log d stages ran). For blocks of 2h polynomials and j < h:
-//   c'[b+j] = c[b+j] + c[b+j+h],  c'[b+j+h] = X^{j d / h} (c[b+j] - c[b+j+h]).
-// With rot_in, input polynomial i is X^i * src[i]. One thread per (pair,
-// coefficient); grid = (ceil(d/2 * d / blockDim), slices).
-template <typename T>
-__global__ void pp_dif_stage_kernel(const T* __restrict__ src, T* __restrict__ dst,
-                                    int d, int log_d, int log_h, int rot_in) {
-  const int64_t cells = static_cast<int64_t>(d / 2) * d;
-  const int64_t cell = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (cell >= cells) return;
-  const int64_t base = static_cast<int64_t>(blockIdx.y) * d * d;
-  const int pr = static_cast<int>(cell >> log_d);
-  const int r = static_cast<int>(cell & (d - 1));
-  const int h = 1 << log_h;
-  const int j = pr & (h - 1);
-  const int i0 = ((pr >> log_h) << (log_h + 1)) + j;
-  const int i1 = i0 + h;
-  const int e = j << (log_d - log_h);  // j d / h < d
-  const T* p0 = src + base + static_cast<int64_t>(i0) * d;
-  const T* p1 = src + base + static_cast<int64_t>(i1) * d;
-  auto load = [&](const T* p, int i, int x) -> T {
-    if (!rot_in) return p[x];
-    return pp_rot_read<T>([&](int y) { return p[y]; }, d, i, x);
-  };
-  const T u = load(p0, i0, r), v = load(p1, i1, r);
-  dst[base + static_cast<int64_t>(i0) * d + r] = static_cast<T>(u + v);
-  const int rr = r >= e ? r - e : r - e + d;
-  const T du = static_cast<T>(load(p0, i0, rr) - load(p1, i1, rr));
-  dst[base + static_cast<int64_t>(i1) * d + r] = r >= e ? du : static_cast<T>(T{0} - du);
-}
+// Where the first pass of a transform reads polynomial i: row i of src as it
+// is; X^i times row i (a_hat_agg); or digit polynomial l of t_vec_g[j]
+// (src_of[i] = 2j) or t_vec_gh[j] (2j + 1), zero for -1
+// (BuildPreprocessMatrix, lwes_to_rlwe.cc:154-172).
+enum PpInput { kPpRows, kPpRotated, kPpDigits };
 
-// Polynomial i of a matrix block before its transform: digit polynomial l of
-// t_vec_g[j] (src_of[i] = 2j) or t_vec_gh[j] (2j + 1), zero for -1
-// (BuildPreprocessMatrix, lwes_to_rlwe.cc:154-172). grid = (ceil(d*d/256), slices).
 template <typename T>
-__global__ void pp_block_input_kernel(const T* __restrict__ tg, const T* __restrict__ tgh,
-                                      const int* __restrict__ src_of, int d, int log_d,
-                                      int k, int l, int64_t chain_stride,
-                                      T* __restrict__ out) {
+struct PpSource {
+  const T* src;       // rows, or t_vec_g
+  const T* tgh;       // kPpDigits: t_vec_gh
+  const int* src_of;  // kPpDigits
+  int64_t chain_stride;
+  int k, l;
+};
+
+// S decimation-in-frequency stages of E[m] = sum_i c[i] X^{2im} (d polynomials
+// of length d per slice; natural order in, bit-reversed order out once all
+// log d stages ran), from half-length h = 2^log_h down. A stage of half-length h
+// maps, for blocks of 2h polynomials and j < h,
+//   c'[b+j] = c[b+j] + c[b+j+h],  c'[b+j+h] = X^{j d / h} (c[b+j] - c[b+j+h]).
+// The pass is bound by memory (each reads and writes d^2 words a slice: 81 us
+// for 8 slices of 2048^2 64-bit words at the copy peak, a radix-2 stage took
+// 87), so it takes as many stages as registers hold: 2^S polynomials q spaced
+// hs = h / 2^(S-1) apart at the P = 2^(S-1) coefficients spaced d / P. With j =
+// j0 + qm hs the rotation of stage s is (j0 d / h) 2^s, the same for the whole
+// upper half, plus qm d / Q (Q = 2^(S-1-s)), a permutation of the P
+// coefficients with signs; the common parts of the stages a polynomial was in
+// the upper half of only add up to where its results go. S = 3 keeps 32 words
+// a thread. grid = (ceil(d^2 / 2^(2S-1) / blockDim), slices).
+template <typename T, int S, PpInput kIn>
+__global__ void __launch_bounds__(256)
+pp_dif_pass_kernel(const PpSource<T> in, T* __restrict__ dst, int d, int log_d, int log_h) {
+  constexpr int kN = 1 << S, kP = 1 << (S - 1);
   const int64_t cell = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (cell >= static_cast<int64_t>(d) * d) return;
-  const int s = blockIdx.y;
-  const int i = static_cast<int>(cell >> log_d), r = static_cast<int>(cell & (d - 1));
-  const int src = __ldg(src_of + i);
-  T v = 0;
-  if (src >= 0) {
-    const T* chain = (src & 1) ? tgh : tg;
-    v = chain[s * chain_stride + (static_cast<int64_t>(src >> 1) * k + l) * d + r];
+  const int log_c = log_d - (S - 1);  // coefficients r < d / P
+  if (cell >= static_cast<int64_t>(d >> S) << log_c) return;
+  const int64_t base = static_cast<int64_t>(blockIdx.y) * d * d;
+  const int r = static_cast<int>(cell & ((1 << log_c) - 1));
+  const int grp = static_cast<int>(cell >> log_c);
+  const int log_hs = log_h - (S - 1);
+  const int j0 = grp & ((1 << log_hs) - 1);
+  const int i0 = ((grp >> log_hs) << (log_h + 1)) + j0;
+  T v[kN][kP];
+#pragma unroll
+  for (int q = 0; q < kN; ++q) {
+    const int i = i0 + (q << log_hs);
+    const T* row;
+    if constexpr (kIn == kPpDigits) {
+      const int from = __ldg(in.src_of + i);
+      row = from < 0 ? nullptr
+                     : ((from & 1) ? in.tgh : in.src) + blockIdx.y * in.chain_stride +
+                           (static_cast<int64_t>(from >> 1) * in.k + in.l) * d;
+    } else {
+      row = in.src + base + static_cast<int64_t>(i) * d;
+    }
+#pragma unroll
+    for (int c = 0; c < kP; ++c) {
+      const int x = r + (c << log_c);
+      if constexpr (kIn == kPpRotated) {
+        v[q][c] = pp_rot_read<T>([&](int y) { return row[y]; }, d, i, x);
+      } else {
+        v[q][c] = kIn == kPpDigits && row == nullptr ? T{0} : row[x];
+      }
+    }
   }
-  out[static_cast<int64_t>(s) * d * d + cell] = v;
+#pragma unroll
+  for (int s = 0; s < S; ++s) {
+    const int Q = 1 << (S - 1 - s);
+#pragma unroll
+    for (int q = 0; q < kN; ++q) {
+      if (q & Q) continue;
+      const int turn = (q & (Q - 1)) * (kP / Q);  // coefficients to rotate by
+      T diff[kP];
+#pragma unroll
+      for (int c = 0; c < kP; ++c) {
+        diff[c] = static_cast<T>(v[q][c] - v[q + Q][c]);
+        v[q][c] = static_cast<T>(v[q][c] + v[q + Q][c]);
+      }
+#pragma unroll
+      for (int c = 0; c < kP; ++c) {
+        v[q + Q][c] = c >= turn ? diff[c - turn] : static_cast<T>(T{0} - diff[c - turn + kP]);
+      }
+    }
+  }
+  const int common = j0 << (log_d - log_h);  // j0 d / h
+#pragma unroll
+  for (int q = 0; q < kN; ++q) {
+    int off = r;
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+      if (q & (1 << (S - 1 - s))) off += common << s;
+    }
+    T* row = dst + base + static_cast<int64_t>(i0 + (q << log_hs)) * d;
+#pragma unroll
+    for (int c = 0; c < kP; ++c) {
+      const int to = (off + (c << log_c)) & (2 * d - 1);  // X^d = -1
+      row[to & (d - 1)] = to & d ? static_cast<T>(T{0} - v[q][c]) : v[q][c];
+    }
+  }
 }
 
 // Column c of block l of the matrix is X^c E[c], E[c] the transform's slot

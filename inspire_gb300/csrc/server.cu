@@ -3765,27 +3765,41 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
         static_cast<const T*>(pa_dev), 0, 0, 2 * k, static_cast<T>(~0ull),
         dW.get<uint32_t>(), d, c);
     RETURN_IF_ERROR(Cuda(cudaGetLastError(), "key part transforms"));
-    // Polynomial transform of d x d words per slice, log d DIF stages from
-    // `in` (rotated on input when rot) ping-ponging through dev0/dev1;
-    // returns the buffer holding the result.
-    auto transform = [&](DevBuf* in, bool rot) -> DevBuf* {
-      DevBuf* src = in;
-      DevBuf* dst = in == &dev0 ? &dev1 : &dev0;
-      const int64_t cells = static_cast<int64_t>(d / 2) * d;
-      const dim3 grid(static_cast<unsigned>((cells + 255) / 256), slices);
-      for (int lh = logd - 1; lh >= 0; --lh) {
-        pp_dif_stage_kernel<T><<<grid, 256, 0, cs>>>(src->get<T>(), dst->get<T>(), d, logd,
-                                                      lh, rot && lh == logd - 1 ? 1 : 0);
-        std::swap(src, dst);
+    // Polynomial transform of d x d words per slice from `in`, ping-ponging
+    // through dev0/dev1: passes of three stages, the first with what is left
+    // over. Returns the buffer holding the result.
+    auto transform = [&](auto first_input, const PpSource<T>& in, DevBuf* dst) -> DevBuf* {
+      PpSource<T> src = in;
+      auto pass = [&](auto stages, auto input, int lh) {
+        constexpr int NS = decltype(stages)::value;
+        const int64_t cells = (static_cast<int64_t>(d) * d) >> (2 * NS - 1);
+        pp_dif_pass_kernel<T, NS, decltype(input)::value>
+            <<<dim3(static_cast<unsigned>((cells + 255) / 256), slices), 256, 0, cs>>>(
+                src, dst->get<T>(), d, logd, lh);
+        src.src = dst->get<T>();
+        dst = dst == &dev0 ? &dev1 : &dev0;
+      };
+      using Rows = std::integral_constant<PpInput, kPpRows>;
+      int lh = logd - 1;
+      const int lead = logd % 3;
+      if (lead == 1) {
+        pass(std::integral_constant<int, 1>{}, first_input, lh);
+      } else if (lead == 2) {
+        pass(std::integral_constant<int, 2>{}, first_input, lh);
+      } else {
+        pass(std::integral_constant<int, 3>{}, first_input, lh);
       }
-      return src;
+      lh -= lead == 0 ? 3 : lead;
+      for (; lh >= 0; lh -= 3) pass(std::integral_constant<int, 3>{}, Rows{}, lh);
+      return dst == &dev0 ? &dev1 : &dev0;
     };
     const dim3 tgrid((d + 31) / 32, (d + 31) / 32, slices);
     pp_atilde_kernel<T><<<tgrid, dim3(32, 8), 0, cs>>>(static_cast<const T*>(hint_dev),
                                                        hint_stride, d, logd, log_modulus,
                                                        dev0.get<T>());
     RETURN_IF_ERROR(Cuda(cudaGetLastError(), "a_tilde"));
-    DevBuf* ev = transform(&dev0, true);
+    DevBuf* ev = transform(std::integral_constant<PpInput, kPpRotated>{},
+                           PpSource<T>{dev0.get<T>(), nullptr, nullptr, 0, 0, 0}, &dev1);
     RETURN_IF_ERROR(Cuda(cudaGetLastError(), "a_hat_agg transform"));
     ChainArgs ca;
     ca.d = d;
@@ -3886,11 +3900,9 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
     }
     // BuildPreprocessMatrix, one d x d block per digit plane l.
     for (int l = 0; l < k; ++l) {
-      const int64_t cells = static_cast<int64_t>(d) * d;
-      pp_block_input_kernel<T><<<dim3(static_cast<unsigned>((cells + 255) / 256), slices), 256,
-                                 0, cs>>>(dtg.get<T>(), dtgh.get<T>(), dsrc.get<int>(), d, logd,
-                                          k, l, chain_stride, dev0.get<T>());
-      DevBuf* mev = transform(&dev0, false);
+      DevBuf* mev = transform(
+          std::integral_constant<PpInput, kPpDigits>{},
+          PpSource<T>{dtg.get<T>(), dtgh.get<T>(), dsrc.get<int>(), chain_stride, k, l}, &dev0);
       switch (mat_kind) {
         case INSPIRE_I16:
           pp_matrix_kernel<T, int16_t><<<tgrid, dim3(32, 8), 0, cs>>>(
