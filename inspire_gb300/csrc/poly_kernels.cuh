@@ -185,6 +185,20 @@ inner_product_finish_kernel(const uint32_t* __restrict__ U,
   }
 }
 
+// Where FinalizeMatrixPack's polynomials go: b of slice s of request q at
+// b[(q slices + s) stride]; with a_tilde the stride is 2 d and the slice's
+// a_tilde_agg (the same for every request) goes right before it, so that the
+// packed ciphertexts come as (a, b) pairs.
+template <typename T>
+struct PackedOut {
+  T* b;
+  int64_t stride;
+  const T* a_tilde;  // [slices][d], or null
+  __device__ __forceinline__ void put_a(int s, int d, int j, T* outp) const {
+    if (a_tilde != nullptr) outp[j - d] = __ldg(a_tilde + static_cast<int64_t>(s) * d + j);
+  }
+};
+
 // FinalizeMatrixPack for every (request, shard, slice):
 //   b_agg = LowBits(LowBits(gemv) + sum_j t_h[j] (*) y_h[j], log_q)
 // gemv already holds b' + b_agg_partial (optionally split in two vectors).
@@ -194,7 +208,7 @@ template <typename T, int ITERS = 0>
 __global__ void __launch_bounds__(PolyShape<ITERS>::kMaxThreads, PolyShape<ITERS>::kMinBlocks)
 finalize_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restrict__ Yh,
                 int k, const T* __restrict__ gemv, const T* __restrict__ gemv2,
-                int64_t gemv_qstride, T* __restrict__ packed_b,
+                int64_t gemv_qstride, PackedOut<T> packed,
                 int log_q, NttCtx c) {
   extern __shared__ uint32_t smem[];  // [r][d]
   const int d = 1 << c.logd;
@@ -215,7 +229,7 @@ finalize_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restrict__ Yh
     ntt_inverse_t<ITERS>(a, c, pi);
   }
   const int64_t base = q * gemv_qstride + static_cast<int64_t>(s) * d;
-  T* outp = packed_b + (static_cast<int64_t>(q) * gridDim.x + s) * d;
+  T* outp = packed.b + (static_cast<int64_t>(q) * gridDim.x + s) * packed.stride;
   for (int j = threadIdx.x; j < d; j += blockDim.x) {
     uint32_t x[kMaxPrimes] = {0, 0, 0, 0, 0};
 #pragma unroll
@@ -229,6 +243,7 @@ finalize_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restrict__ Yh
     T g = gemv[base + j];
     if (gemv2 != nullptr) g += gemv2[base + j];
     outp[j] = low_bits<T>(static_cast<T>(low_bits<T>(g, log_q) + inner), log_q);
+    packed.put_a(s, d, j, outp);
   }
 }
 
@@ -242,7 +257,7 @@ template <typename T, int LOGD>
 __global__ void __launch_bounds__(Ntt16<LOGD>::kThreads, 512 / Ntt16<LOGD>::kThreads)
 finalize16_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restrict__ Yh,
                   int k, const T* __restrict__ gemv, const T* __restrict__ gemv2,
-                  int64_t gemv_qstride, T* __restrict__ packed_b, int log_q,
+                  int64_t gemv_qstride, PackedOut<T> packed, int log_q,
                   NttCtx c) {
   extern __shared__ uint32_t smem[];  // exchange buffer, then [r][d] results
   constexpr int d = Ntt16<LOGD>::kD;
@@ -280,7 +295,7 @@ finalize16_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restrict__ 
     }
   }
   const int64_t base = q * gemv_qstride + static_cast<int64_t>(s) * d;
-  T* outp = packed_b + (static_cast<int64_t>(q) * gridDim.x + s) * d;
+  T* outp = packed.b + (static_cast<int64_t>(q) * gridDim.x + s) * packed.stride;
   for (int jj = 0; jj < 16; ++jj) {
     const int j = tid + NT * jj;
     uint32_t x[kMaxPrimes] = {0, 0, 0, 0, 0};
@@ -292,6 +307,7 @@ finalize16_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restrict__ 
     T g = gemv[base + j];
     if (gemv2 != nullptr) g += gemv2[base + j];
     outp[j] = low_bits<T>(static_cast<T>(low_bits<T>(g, log_q) + inner), log_q);
+    packed.put_a(s, d, j, outp);
   }
 }
 
@@ -306,7 +322,7 @@ template <typename T, int LOGD, int NGR = 2>
 __global__ void __launch_bounds__(NGR * Ntt16<LOGD>::kThreads, 1)
 finalize16_pair_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restrict__ Yh,
                        int k, const T* __restrict__ gemv, const T* __restrict__ gemv2,
-                       int64_t gemv_qstride, T* __restrict__ packed_b, int log_q,
+                       int64_t gemv_qstride, PackedOut<T> packed, int log_q,
                        NttCtx c) {
   extern __shared__ uint32_t smem[];
   constexpr int d = Ntt16<LOGD>::kD;
@@ -357,7 +373,7 @@ finalize16_pair_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restri
   }
   __syncthreads();
   const int64_t base = q * gemv_qstride + static_cast<int64_t>(s) * d;
-  T* outp = packed_b + (static_cast<int64_t>(q) * gridDim.x + s) * d;
+  T* outp = packed.b + (static_cast<int64_t>(q) * gridDim.x + s) * packed.stride;
 #pragma unroll 4
   for (int j = tid; j < d; j += NGR * NT) {
     uint32_t x[kMaxPrimes] = {0, 0, 0, 0, 0};
@@ -369,23 +385,7 @@ finalize16_pair_kernel(const uint32_t* __restrict__ Th, const uint32_t* __restri
     T g = gemv[base + j];
     if (gemv2 != nullptr) g += gemv2[base + j];
     outp[j] = low_bits<T>(static_cast<T>(low_bits<T>(g, log_q) + inner), log_q);
-  }
-}
-
-// The packed ciphertexts as (a_tilde_agg, b_agg) pairs:
-// out[q][s] = (a[s], b[q][s]). grid = (shards, batch).
-template <typename T>
-__global__ void __launch_bounds__(kPolyThreads)
-pack_out_kernel(const T* __restrict__ a, const T* __restrict__ b, int d,
-                T* __restrict__ out) {
-  const int s = blockIdx.x;
-  const int64_t qs = static_cast<int64_t>(blockIdx.y) * gridDim.x + s;
-  const T* as = a + static_cast<int64_t>(s) * d;
-  const T* bs = b + qs * d;
-  T* o = out + qs * 2 * d;
-  for (int j = threadIdx.x; j < d; j += blockDim.x) {
-    o[j] = as[j];
-    o[d + j] = bs[j];
+    packed.put_a(s, d, j, outp);
   }
 }
 

@@ -29,6 +29,7 @@
 #include "limb_gemm.h"
 #include "ntt.cuh"
 #include "answer_poly.cuh"
+#include "ext_product.cuh"
 #include "hint16.cuh"
 #include "poly_kernels.cuh"
 #include "preprocess_kernels.cuh"
@@ -582,6 +583,7 @@ struct inspire_pir_server {
   inspire::NttCtx ctx_f{}, ctx_e{};
   bool fused_poly = false;  // answers run answer_poly_kernel
   inspire::CrtArgs crt{};   // its reconstruction constants
+  bool fused_ext = false;   // batched ExternalProduct runs ext_product_kernel
   uint64_t vmask_f = 0, vmask_e = 0, umask_e = 0;
   std::unique_ptr<inspire::LimbGemm> limb;
 
@@ -747,7 +749,7 @@ Status LaunchPairExt(int64_t blocks, int sms, dim3 grid, cudaStream_t st, A... a
 template <typename T, int LG>
 Status LaunchPairFinalize(const NttCtx& c, dim3 grid, cudaStream_t st, const uint32_t* th,
                           const uint32_t* yh, int k, const T* gemv, int64_t rows,
-                          T* packed, int log_q) {
+                          PackedOut<T> packed, int log_q) {
   constexpr int d = Ntt16<LG>::kD;
   if constexpr (LG <= 11) {
     if (c.r >= 3) {
@@ -797,12 +799,16 @@ Status RgswTransform(inspire_pir_server* s, Workspace* w, int batch, const T* sd
 }
 
 // yh_done: the y_h transform is already in w->yh (enqueued on another
-// stream that `st` has joined).
+// stream that `st` has joined). pairs: write (a_tilde_agg, b_agg) pairs there
+// instead of the b polynomials to w->packed.
 template <typename T>
 Status FinalizeStage(inspire_pir_server* s, Workspace* w, int batch,
                      const T* pkey, const T* gemv, cudaStream_t st,
-                     bool yh_done = false) {
+                     bool yh_done = false, T* pairs = nullptr) {
   const int d = s->d, t = s->t, l = s->l, k = s->k;
+  const PackedOut<T> packed =
+      pairs == nullptr ? PackedOut<T>{w->packed.get<T>(), d, nullptr}
+                       : PackedOut<T>{pairs + d, int64_t{2} * d, s->a_tilde.get<T>()};
   const int log_q = s->prm.log_modulus;
   if (!yh_done) RETURN_IF_ERROR(YhTransform<T>(s, w, batch, pkey, st));
   if (s->ctx_f.tables16 != nullptr && static_cast<int64_t>(l) * t * batch >= s->sms) {
@@ -812,7 +818,7 @@ Status FinalizeStage(inspire_pir_server* s, Workspace* w, int batch,
         c.logd, RETURN_IF_ERROR(SetSmem(finalize16_kernel<T, LG>, smem));
         finalize16_kernel<T, LG><<<dim3(l * t, batch), Ntt16<LG>::kThreads, smem, st>>>(
             s->th_ntt.get<uint32_t>(), w->yh.get<uint32_t>(), k, gemv, nullptr, s->rows,
-            w->packed.get<T>(), log_q, c));
+            packed, log_q, c));
     RETURN_IF_ERROR(Cuda(cudaGetLastError(), "finalize"));
   } else if (s->ctx_f.tables16 != nullptr && d <= 4096) {
     // Several transform groups per block.
@@ -820,7 +826,7 @@ Status FinalizeStage(inspire_pir_server* s, Workspace* w, int batch,
     INSPIRE_NTT16_PAIR_DISPATCH(
         c.logd, RETURN_IF_ERROR((LaunchPairFinalize<T, LG>(
                     c, dim3(l * t, batch), st, s->th_ntt.get<uint32_t>(),
-                    w->yh.get<uint32_t>(), k, gemv, s->rows, w->packed.get<T>(), log_q))));
+                    w->yh.get<uint32_t>(), k, gemv, s->rows, packed, log_q))));
   } else {
     const NttCtx& c = s->ctx_f;
     const size_t smem = static_cast<size_t>(c.r) * d * 4;
@@ -830,7 +836,7 @@ Status FinalizeStage(inspire_pir_server* s, Workspace* w, int batch,
         pl.iters, RETURN_IF_ERROR(SetSmem(finalize_kernel<T, IT>, smem));
         finalize_kernel<T, IT><<<grid, pl.nt, smem, st>>>(
             s->th_ntt.get<uint32_t>(), w->yh.get<uint32_t>(), k, gemv, nullptr, s->rows,
-            w->packed.get<T>(), log_q, c));
+            packed, log_q, c));
     RETURN_IF_ERROR(Cuda(cudaGetLastError(), "finalize"));
   }
   return Status{};
@@ -1224,13 +1230,55 @@ Status PackOnDevice(inspire_pir_server* s, Workspace* w, int batch,
   RETURN_IF_ERROR(Products(s, w, batch, q1, pkey, w->gemv.get(), engine, st));
   auto run = [&](auto tag) -> Status {
     using T = decltype(tag);
-    RETURN_IF_ERROR(FinalizeStage<T>(s, w, batch, static_cast<const T*>(pkey),
-                                     w->gemv.get<T>(), st));
-    pack_out_kernel<T><<<dim3(s->l * s->t, batch), PolyThreads(s->d), 0, st>>>(
-        s->a_tilde.get<T>(), w->packed.get<T>(), s->d, static_cast<T*>(out));
-    return Cuda(cudaGetLastError(), "pack output");
+    return FinalizeStage<T>(s, w, batch, static_cast<const T*>(pkey), w->gemv.get<T>(), st,
+                            false, static_cast<T*>(out));
   };
   return s->prm.coeff_bits == 32 ? run(uint32_t{}) : run(uint64_t{});
+}
+
+// Launches ext_product_kernel.
+template <typename T, int LOGD, int G, bool kOne>
+Status LaunchExtProduct(const ExtProductArgs<T>& a, int batch, cudaStream_t st) {
+  constexpr int R = AnswerPolyPrimes<T>();
+  constexpr size_t smem = ExtProductSmem<T, LOGD, G>();
+  auto* kernel = ext_product_kernel<T, LOGD, G, kOne, R>;
+  RETURN_IF_ERROR(SetSmem(kernel, smem));
+  cudaLaunchAttribute cluster;
+  cluster.id = cudaLaunchAttributeClusterDimension;
+  cluster.val.clusterDim.x = R;
+  cluster.val.clusterDim.y = 1;
+  cluster.val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(R, batch);
+  cfg.blockDim = dim3(G * Ntt16<LOGD>::kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = &cluster;
+  cfg.numAttrs = 1;
+  return Cuda(cudaLaunchKernelEx(&cfg, kernel, a), "external product");
+}
+
+// The batched external product in one launch (ext_product.cuh): a group per
+// live digit up to four (d = 2048) or, at 256 threads a group and two
+// residue sums in registers, two groups in turns.
+template <typename T>
+Status FusedExtProduct(inspire_pir_server* s, int batch, const T* ct, const T* rgsw, T* out,
+                       cudaStream_t st) {
+  ExtProductArgs<T> a;
+  a.ct = ct;
+  a.rgsw = rgsw;
+  a.out = out;
+  a.vmask = static_cast<T>(s->vmask_e);
+  a.e = ExtArgs{s->prm.log_modulus, s->prm.eval_log_digit, s->ne,
+                LiveDigits(s->prm.log_modulus, s->prm.eval_log_digit, s->ne), s->umask_e};
+  a.crt = s->crt;
+  a.c = s->ctx_e;
+  const bool one = 2 * a.e.live_digits <= 4;
+  if (s->d == 2048) {
+    return one ? LaunchExtProduct<T, 11, 4, true>(a, batch, st)
+               : LaunchExtProduct<T, 11, 3, false>(a, batch, st);
+  }
+  return LaunchExtProduct<T, 12, 2, false>(a, batch, st);
 }
 
 // ExternalProduct (external_product.cc:35-114) of `batch` independent
@@ -1241,6 +1289,15 @@ Status ExternalOnDevice(inspire_pir_server* s, Workspace* w, int batch,
                         const void* ct, const void* rgsw, void* out,
                         cudaStream_t st) {
   RETURN_IF_ERROR(s->eval_rule);
+  if (s->fused_ext) {
+    return s->prm.coeff_bits == 32
+               ? FusedExtProduct<uint32_t>(s, batch, static_cast<const uint32_t*>(ct),
+                                           static_cast<const uint32_t*>(rgsw),
+                                           static_cast<uint32_t*>(out), st)
+               : FusedExtProduct<uint64_t>(s, batch, static_cast<const uint64_t*>(ct),
+                                           static_cast<const uint64_t*>(rgsw),
+                                           static_cast<uint64_t*>(out), st);
+  }
   const int d = s->d, ne = s->ne, ng = 2 * s->ne;
   const NttCtx& c = s->ctx_e;
   const size_t need = static_cast<size_t>(batch) * ng * c.r * d * 4;
@@ -1539,6 +1596,10 @@ Status CreateServer(const inspire_pir_params* prm, const void* db,
     }
   }
   // The server's calls come on streams of their own: wait for the tables.
+  if (set == kSet27 && d <= 4096 && se.ok()) {
+    s->fused_ext =
+        r_e <= (cb == 32 ? AnswerPolyPrimes<uint32_t>() : AnswerPolyPrimes<uint64_t>());
+  }
   RETURN_IF_ERROR(NttTables::Create(prm->log_degree, set, nullptr, &s->tables, false));
   RETURN_IF_ERROR(Cuda(cudaStreamSynchronize(nullptr), "NTT tables"));
   {
@@ -1548,7 +1609,10 @@ Status CreateServer(const inspire_pir_params* prm, const void* db,
     }
   }
   s->ctx_f = s->tables->Ctx(r_f);
-  if (s->fused_poly) s->crt = s->tables->Crt(r_f);
+  if (s->fused_poly || s->fused_ext) {
+    s->crt = s->tables->Crt(cb == 32 ? AnswerPolyPrimes<uint32_t>()
+                                     : AnswerPolyPrimes<uint64_t>());
+  }
   s->ctx_e = s->tables->Ctx(r_e);
 
   const size_t w = Words(cb);
@@ -4206,7 +4270,7 @@ int inspire_finalize_matrix_pack(const inspire_pir_params* params,
     RETURN_IF_ERROR(SetSmem(finalize_kernel<T>, smem));
     finalize_kernel<T><<<dim3(1, 1), kPolyThreads, smem>>>(
         dTh.get<uint32_t>(), dYh.get<uint32_t>(), k, db1.get<T>(), db2.get<T>(), 0,
-        dout.get<T>(), params->log_modulus, c);
+        PackedOut<T>{dout.get<T>(), d, nullptr}, params->log_modulus, c);
     return Cuda(cudaDeviceSynchronize(), "finalize");
   };
   if (st.ok()) st = cb == 32 ? run(uint32_t{}) : run(uint64_t{});
