@@ -149,17 +149,29 @@ interpolate_kernel(const V* __restrict__ raw, InterpArgs a, V* __restrict__ out)
 constexpr int kFastR = 32;   // classes per block (one warp's lanes)
 // Groups per block (kG: the stores run over kG consecutive columns) and
 // groups in flight (kGW warps per block). 8- and 16-bit values take 32
-// groups (64-byte row pieces; an 80 KB tile of 16-bit values at t = 8, two
+// groups (64-byte row pieces; a 64 KB tile of 16-bit values at t = 8, two
 // blocks per SM, as the registers of the t = 8 transform allow); wider
 // values 16, which keeps the tile within a block's limit.
 template <typename V>
 struct FastShape {
   static constexpr int kG = sizeof(V) <= 2 ? 32 : 16;
   static constexpr int kGW = 8;
-  // Tile row pitch in values: padded against bank conflicts; for 16-bit
-  // values 40 (80-byte rows), so that eight neighbouring groups read as one
-  // 16-byte vector.
-  static constexpr int kRow = kG + (sizeof(V) == 2 ? 8 : 1);
+  // Tile row pitch in values, padded against bank conflicts; 16-bit rows (16
+  // words) are permuted instead: word w of class c sits at w ^ (c / 2), so 32
+  // classes' writes of one word and the store phase's reads of consecutive
+  // words both touch 32 banks. (Padded to 80 bytes for 16-byte reads, the
+  // writes took four passes each.)
+  static constexpr int kRow = sizeof(V) == 2 ? kG : kG + 1;
+  __device__ static __forceinline__ int swizzle(int c) { return (c >> 1) & 15; }
+  // Index of (tile row rm, class c, group g).
+  __device__ static __forceinline__ int at(int rm, int c, int g) {
+    const int row = rm * kFastR + c;
+    if constexpr (sizeof(V) == 2) {
+      return row * kRow + 2 * ((g >> 1) ^ swizzle(c)) + (g & 1);
+    } else {
+      return row * kRow + g;
+    }
+  }
 };
 
 // Modular helpers; SMALL: p < 2^31, so sums and Shoup remainders fit in 32
@@ -291,18 +303,17 @@ __device__ __forceinline__ void lazy_transform(uint32_t (&x)[T][T / 2], const In
 
 // Writes the transformed subproblems of groups gi (xa) and gi + 1 (xb, when
 // hb) of class c0 to the block's tile; 16-bit values of the two groups go as
-// one 32-bit word (gi even, even row pitch).
+// one 32-bit word (gi even).
 template <typename V, int T>
 __device__ __forceinline__ void lazy_tile_store(const uint32_t (&xa)[T][T / 2],
                                                 const uint32_t (&xb)[T][T / 2], bool hb,
                                                 int gi, int c0, V* tile) {
   constexpr int H = T / 2;
-  constexpr int kRow = FastShape<V>::kRow;
 #pragma unroll
   for (int r = 0; r < T; ++r) {
 #pragma unroll
     for (int m = 0; m < H; ++m) {
-      V* dst = tile + ((r * H + m) * kFastR + c0) * kRow + gi;
+      V* dst = tile + FastShape<V>::at(r * H + m, c0, gi);
       if constexpr (sizeof(V) == 2) {
         if (hb) {
           *reinterpret_cast<uint32_t*>(dst) = xa[r][m] | (xb[r][m] << 16);
@@ -332,10 +343,9 @@ interpolate_fast_kernel(const V* __restrict__ raw, InterpArgs a, ModConsts mc,
   constexpr int LOGT = T == 2 ? 1 : (T == 4 ? 2 : 3);
   constexpr int kFastG = FastShape<V>::kG;
   constexpr int kFastGW = FastShape<V>::kGW;
-  // [T*H rows][kFastR classes][kFastG + 1 groups] (dynamic shared memory)
+  // [T*H rows][kFastR classes][groups] (dynamic shared memory)
   extern __shared__ __align__(16) unsigned char tile_raw[];
   V* tile = reinterpret_cast<V*>(tile_raw);
-  constexpr int kRow = FastShape<V>::kRow;
   const int c0 = threadIdx.x % kFastR;
   const int gw = threadIdx.x / kFastR;
   // Class blocks fastest: blocks running together read neighbouring 64-byte
@@ -415,7 +425,7 @@ interpolate_fast_kernel(const V* __restrict__ raw, InterpArgs a, ModConsts mc,
     for (int r = 0; r < T; ++r) {
 #pragma unroll
       for (int m = 0; m < H; ++m) {
-        tile[((r * H + m) * kFastR + c0) * kRow + gi] =
+        tile[FastShape<V>::at(r * H + m, c0, gi)] =
             static_cast<V>(scale_p<SMALL>(x[r][m], a.tinv, p, mc));
       }
     }
@@ -429,8 +439,8 @@ interpolate_fast_kernel(const V* __restrict__ raw, InterpArgs a, ModConsts mc,
     if ((a.out_cols & 7) == 0 && G == kFastG &&
         (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
       // Eight neighbouring groups per 16-byte store: four lanes write one
-      // DB row's 64 bytes, a warp eight rows per instruction (row pitch a
-      // multiple of 8 values, g_base a multiple of 32). Thread i writes
+      // DB row's 64 bytes, a warp eight rows per instruction (g_base a
+      // multiple of 32). Thread i writes
       // chunk i % 4 of class (i / 4) % 32, tile rows i / 128 + 2 j.
       constexpr int kChunks = kFastG / 8;
       constexpr int kThreads = kFastR * kFastGW;
@@ -445,20 +455,23 @@ interpolate_fast_kernel(const V* __restrict__ raw, InterpArgs a, ModConsts mc,
       const int64_t ss = static_cast<int64_t>(a.s) * a.out_cols;
       V* dst = out + (static_cast<int64_t>(k) * T * a.d + c_start + c) * a.out_cols + g_base +
                8 * q;
-      const V* src = tile + c * kRow + 8 * q;
+      const uint32_t* src = reinterpret_cast<const uint32_t*>(tile) + c * (kFastG / 2);
+      const int swz = FastShape<V>::swizzle(c);
 #pragma unroll
       for (int j = 0; j < kIters; ++j) {
         const int rm = rm0 + kRmStep * j;
         const int r = rm / H, m = rm % H;
-        const uint4 v = *reinterpret_cast<const uint4*>(src + rm * kFastR * kRow);
+        const uint32_t* w = src + rm * kFastR * (kFastG / 2);
+        const uint4 v = make_uint4(w[(4 * q) ^ swz], w[(4 * q + 1) ^ swz],
+                                   w[(4 * q + 2) ^ swz], w[(4 * q + 3) ^ swz]);
         *reinterpret_cast<uint4*>(dst + r * ds + m * ss) = v;
       }
       return;
     }
     if ((a.out_cols & 1) == 0 && G == kFastG &&
         (reinterpret_cast<uintptr_t>(out) & 3) == 0) {
-      // Two neighbouring groups per 32-bit store (even row pitch, g_base a
-      // multiple of 32: every store is 4-byte aligned).
+      // Two neighbouring groups per 32-bit store (g_base a multiple of 32:
+      // every store is 4-byte aligned).
       constexpr int kPairs = kFastG / 2;
       for (int idx = threadIdx.x; idx < T * H * kFastR * kPairs; idx += blockDim.x) {
         const int gp = idx % kPairs;
@@ -469,7 +482,7 @@ interpolate_fast_kernel(const V* __restrict__ raw, InterpArgs a, ModConsts mc,
                             static_cast<int64_t>(r) * a.d + c_start + c +
                             static_cast<int64_t>(m) * a.s;
         const uint32_t v =
-            *reinterpret_cast<const uint32_t*>(tile + (rm * kFastR + c) * kRow + 2 * gp);
+            *reinterpret_cast<const uint32_t*>(tile + FastShape<V>::at(rm, c, 2 * gp));
         *reinterpret_cast<uint32_t*>(out + row * a.out_cols + g_base + 2 * gp) = v;
       }
       return;
@@ -483,7 +496,7 @@ interpolate_fast_kernel(const V* __restrict__ raw, InterpArgs a, ModConsts mc,
     const int r = rm / H, m = rm % H;
     const int64_t row = static_cast<int64_t>(k) * T * a.d + static_cast<int64_t>(r) * a.d +
                         c_start + c + static_cast<int64_t>(m) * a.s;
-    out[row * a.out_cols + g_base + g] = tile[(rm * kFastR + c) * kRow + g];
+    out[row * a.out_cols + g_base + g] = tile[FastShape<V>::at(rm, c, g)];
   }
 }
 
