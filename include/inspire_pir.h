@@ -262,7 +262,8 @@ int inspire_pir_external_product_device(inspire_pir_server* server,
  * Autotuner of the tensor engine (no reference counterpart): times the
  * batched product for `batch` requests on this server's matrices in every
  * available form (resident digit planes or the DB as stored), request tile
- * (64 requests, 32 over Z_2^64; or 16, tried up to 64 requests) and split-K
+ * (the multiple of 16 up to 64 requests that takes the batch in as few tiles
+ * as 64 do, 32 over Z_2^64; or 16, tried up to 64 requests) and split-K
  * factor, and keeps the fastest for later batches of the same size
  * (rounded up to 16 requests). Reports the split-K factor and the product's
  * time in ms. Synchronous; FAILED_PRECONDITION without the tensor engine.

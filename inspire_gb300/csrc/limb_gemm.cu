@@ -118,18 +118,18 @@ static_assert(kSmemBytes <= 227 * 1024, "shared memory per CTA");
 // fit: 9 with narrow request tiles) that
 // the producer fills ahead of the converter, so that a raw tile is already
 // on chip when its box frees up.
-// Full request tiles leave no room for staging: their converting form loads
-// each raw tile into the first half of its own box (once the MMA pipe has
-// freed it) and the converter expands it in place.
+// Request tiles of 32 and more leave no room for eight staging slots: their
+// converting form loads each raw tile into the first half of its own box (once
+// the MMA pipe has freed it) and the converter expands it in place.
 constexpr int kMaxStages = 16;  // staging slots the barrier region provides for
 template <int NQ, bool CONV, int TQ>
 struct RingPlan {
   static constexpr int kBSlotB = NQ * TQ * kBSlotK * 2;
-  static constexpr bool kStaged = CONV && NQ * TQ < kBRows;
   static constexpr int kBS = kBSlots;
   static constexpr int kBBase = kRowBlocks * kARingBytes;
   static constexpr int kStageBase = kBBase + kBS * kBSlotB;
   static constexpr int kFree = (kRingBytes - kStageBase) / kRawTileBytes;
+  static constexpr bool kStaged = CONV && kFree >= 8;
   static constexpr int kStages = kStaged ? (kFree < kMaxStages ? kFree : kMaxStages) : 0;
   static_assert(!kStaged || kStages >= 4, "raw staging ring");
   // The converter warps' parity waits on the staging slots are exact when
@@ -147,7 +147,9 @@ struct RingPlan {
 // requests) cuts the MMA work of small batches by 256 / (16 NQ): the DB is
 // then streamed once per 16 requests instead of once per 64 (or 32) padded
 // ones, with N = 16 NQ, ..., 16 (NQ - 3), all multiples of 16 as M = 128
-// needs.
+// needs. Over Z_2^32 there are tiles of 32 and 48 too, for batches that fill
+// a full tile to half or three quarters: the tensor work, the decoding and
+// the request loads go with the tile.
 template <int NQ>
 struct LimbShape {
   using Acc = typename std::conditional<NQ == 4, uint32_t, unsigned long long>::type;
@@ -804,7 +806,7 @@ limb_gemm_kernel(const __grid_constant__ CUtensorMap tm_db,
 #pragma unroll
       for (int sblk = 0; sblk < NW; ++sblk) {
         if (kind == 2 && sblk < 2) continue;
-        constexpr int kLd = kTileQ < 32 ? kTileQ : 32;  // columns per load
+        constexpr int kLd = kTileQ % 32 == 0 ? 32 : 16;  // columns per load
         uint32_t v[kTileQ / kLd][kLd];
 #pragma unroll
         for (int c = 0; c < kTileQ / kLd; ++c) {
@@ -1082,8 +1084,7 @@ class LimbScratchImpl : public LimbScratch {
   __half* q_planes = nullptr;
   __half* y_planes = nullptr;
   void* qsum = nullptr;  // sum_c q1[q][c] per request (coefficient words)
-  CUtensorMap tm_q{}, tm_y{};      // boxes of a full request tile
-  CUtensorMap tm_qn{}, tm_yn{};    // boxes of a narrow tile
+  CUtensorMap tm_q[4]{}, tm_y[4]{};  // boxes of 16, 32, 48 and 64 requests
 };
 
 class LimbGemmImpl : public LimbGemm {
@@ -1139,9 +1140,13 @@ class LimbGemmImpl : public LimbGemm {
     };
     if (nq == 4) {
       allow(reinterpret_cast<const void*>(limb_gemm_kernel<4, false, 64>));
+      allow(reinterpret_cast<const void*>(limb_gemm_kernel<4, false, 48>));
+      allow(reinterpret_cast<const void*>(limb_gemm_kernel<4, false, 32>));
       allow(reinterpret_cast<const void*>(limb_gemm_kernel<4, false, kNarrowTQ>));
       if (conv_) {
         allow(reinterpret_cast<const void*>(limb_gemm_kernel<4, true, 64>));
+        allow(reinterpret_cast<const void*>(limb_gemm_kernel<4, true, 48>));
+        allow(reinterpret_cast<const void*>(limb_gemm_kernel<4, true, 32>));
         allow(reinterpret_cast<const void*>(limb_gemm_kernel<4, true, kNarrowTQ>));
       }
     } else {
@@ -1184,15 +1189,14 @@ class LimbGemmImpl : public LimbGemm {
     if (e != cudaSuccess) return e;
     e = cudaMalloc(&sc->qsum, static_cast<size_t>(word_) * need);
     if (e != cudaSuccess) return e;
-    if (!make_map(&sc->tm_q, sc->q_planes, static_cast<uint64_t>(nq_) * need, cpad_, tq_,
-                  kBSlotK) ||
-        !make_map(&sc->tm_y, sc->y_planes, static_cast<uint64_t>(nq_) * need, kpad_, tq_,
-                  kBSlotK) ||
-        !make_map(&sc->tm_qn, sc->q_planes, static_cast<uint64_t>(nq_) * need, cpad_,
-                  kNarrowTQ, kBSlotK) ||
-        !make_map(&sc->tm_yn, sc->y_planes, static_cast<uint64_t>(nq_) * need, kpad_,
-                  kNarrowTQ, kBSlotK)) {
-      return cudaErrorInvalidValue;
+    for (int tq = kNarrowTQ; tq <= tq_; tq += kNarrowTQ) {
+      const int i = tq / kNarrowTQ - 1;
+      if (!make_map(&sc->tm_q[i], sc->q_planes, static_cast<uint64_t>(nq_) * need, cpad_, tq,
+                    kBSlotK) ||
+          !make_map(&sc->tm_y[i], sc->y_planes, static_cast<uint64_t>(nq_) * need, kpad_, tq,
+                    kBSlotK)) {
+        return cudaErrorInvalidValue;
+      }
     }
     sc->qcap = need;
     return cudaSuccess;
@@ -1210,7 +1214,7 @@ class LimbGemmImpl : public LimbGemm {
                       cudaStream_t st, int form, int split, int out_bits) override {
     Choice c = Chosen(batch);
     c.form = form & 1;
-    c.narrow = (form >> 1) & 1;
+    c.tq = (form >> 1) & 1 ? kNarrowTQ : tq_;
     if (split > 0) c.split = split;
     if (!Available(c)) return cudaErrorNotSupported;
     return Launch(batch, q1, q1_stride, yg, yg_stride, out, scratch, st, c,
@@ -1224,15 +1228,24 @@ class LimbGemmImpl : public LimbGemm {
     return nq_ == 8 && out_bits > 0 && out_bits <= 56 ? 7 : nq_;
   }
 
-  // One configuration of the product: split-K factor, DB form and request
-  // tile (1: the narrow 16-request tile).
+  // One configuration of the product: split-K factor, DB form and requests
+  // per tile.
   struct Choice {
-    int split, form, narrow;
+    int split, form, tq;
   };
 
   bool Available(const Choice& c) const {
-    if (c.narrow && nq_ != 4) return false;
+    if (c.tq != tq_ && nq_ != 4) return false;
     return (c.form == kFormRaw && conv_) || (c.form == kFormPlanes && db_planes_);
+  }
+
+  // The smallest request tile that takes the batch in as many tiles as full
+  // ones do (the DB is streamed once per tile): less padding at no more DB
+  // traffic.
+  int FitTile(int batch) const {
+    if (nq_ != 4) return tq_;
+    const int tiles = (batch + tq_ - 1) / tq_;
+    return static_cast<int>(round_up((batch + tiles - 1) / tiles, kNarrowTQ));
   }
 
   // Tuned choices are kept per batch size rounded up to the narrow tile.
@@ -1241,7 +1254,8 @@ class LimbGemmImpl : public LimbGemm {
   // Autotuner: times every available (form, request tile, split-K factor)
   // with at least 8 K units per CTA and 80 % of the last wave busy (plus the
   // heuristic factor) on this batch size, and keeps the fastest for later
-  // launches of the same size. The narrow tile is tried up to 64 requests.
+  // launches of the same size. Tried are the tile that fits (FitTile) and, up
+  // to 64 requests, the narrow one.
   // Synchronises `st`.
   cudaError_t Tune(int batch, const void* q1, int64_t q1_stride, const void* yg,
                    int64_t yg_stride, void* out, LimbScratch* scratch,
@@ -1261,14 +1275,14 @@ class LimbGemmImpl : public LimbGemm {
     }
     Choice best = Heuristic(batch);
     float best_t = 0;
-    for (int narrow = 0; narrow <= (batch <= 64 && nq_ == 4 ? 1 : 0) && e == cudaSuccess;
-         ++narrow) {
-      const int tq = narrow ? kNarrowTQ : tq_;
+    const int fit = FitTile(batch);
+    for (int tq = tq_; tq >= kNarrowTQ && e == cudaSuccess; tq -= kNarrowTQ) {
+      if (tq != fit && !(tq == kNarrowTQ && batch <= 64 && nq_ == 4)) continue;
       const int64_t tiles = (rows_ / kTileRows) * ((batch + tq - 1) / tq);
       const int heuristic = ChooseSplit(tiles, n_units);
       for (int form = kFormPlanes; form <= kFormRaw && e == cudaSuccess; ++form) {
         for (int k = 1; k <= 16 && e == cudaSuccess; ++k) {
-          const Choice c{k, form, narrow};
+          const Choice c{k, form, tq};
           if (!Available(c)) break;
           if (n_units / k < 8) break;
           const int64_t items = tiles * k;
@@ -1299,18 +1313,22 @@ class LimbGemmImpl : public LimbGemm {
       tuned_[TuneKey(batch)] = best;
     }
     if (chosen) *chosen = best.split;
-    if (chosen_form) *chosen_form = best.form + 2 * best.narrow;
+    if (chosen_form) *chosen_form = best.form + (best.tq == kNarrowTQ ? 2 : 0);
     if (best_ms) *best_ms = best_t / 2;
     return cudaSuccess;
   }
 
-  // Without a tuned choice: the full tile, the resident planes when there
-  // are some (the form measured fastest for large batches), else the DB as
-  // stored, and the split-K factor that fills the SMs.
+  // Without a tuned choice: the tile that fits; the DB as stored up to 64
+  // requests and the resident planes beyond (where each was measured faster:
+  // 2.2 against 2.8 ms up to 16 requests, 3.1 against 3.2 at 64, 5.9 against
+  // 5.0 at 128 on 32768 x 131072 u16); and the split-K factor that fills the
+  // SMs.
   Choice Heuristic(int batch) const {
-    const int64_t tiles = (rows_ / kTileRows) * ((batch + tq_ - 1) / tq_);
+    const int tq = FitTile(batch);
+    const int64_t tiles = (rows_ / kTileRows) * ((batch + tq - 1) / tq);
+    const bool raw = conv_ && (batch <= 64 || !db_planes_);
     return {ChooseSplit(tiles, static_cast<int>((cpad_ + 2 * kpad_) / kUnitK)),
-            db_planes_ ? kFormPlanes : kFormRaw, 0};
+            raw ? kFormRaw : kFormPlanes, tq};
   }
 
   Choice Chosen(int batch) {
@@ -1359,15 +1377,15 @@ class LimbGemmImpl : public LimbGemm {
     a.batch = batch;
     a.out_stride = rows_;
     a.ksplit = c.split;
-    const int tq = c.narrow ? kNarrowTQ : tq_;
+    const int tq = c.tq;
     const int64_t tiles = (rows_ / kTileRows) * ((batch + tq - 1) / tq);
     if (a.ksplit > 1) {
       e = cudaMemsetAsync(out, 0, static_cast<size_t>(batch) * rows_ * word_, st);
       if (e != cudaSuccess) return e;
     }
     const unsigned grid = static_cast<unsigned>(tiles * a.ksplit);
-    const CUtensorMap& mq = c.narrow ? sc->tm_qn : sc->tm_q;
-    const CUtensorMap& my = c.narrow ? sc->tm_yn : sc->tm_y;
+    const CUtensorMap& mq = sc->tm_q[tq / kNarrowTQ - 1];
+    const CUtensorMap& my = sc->tm_y[tq / kNarrowTQ - 1];
     using U = unsigned long long;
     const uint32_t* qs4 = static_cast<const uint32_t*>(sc->qsum);
     const U* qs8 = static_cast<const U*>(sc->qsum);
@@ -1379,10 +1397,17 @@ class LimbGemmImpl : public LimbGemm {
   limb_gemm_kernel<NQ, CONV, TQ, NW><<<grid, nt, kSmemBytes, st>>>(                 \
       tm_db_, tm_raw_, tm_pk_, mq, my, a, QS, OUT, err_)
     if (nq_ == 4) {
-      if (!raw && !c.narrow) INSPIRE_LIMB_LAUNCH(4, false, 64, 4, qs4, o4);
-      if (!raw && c.narrow) INSPIRE_LIMB_LAUNCH(4, false, kNarrowTQ, 4, qs4, o4);
-      if (raw && !c.narrow) INSPIRE_LIMB_LAUNCH(4, true, 64, 4, qs4, o4);
-      if (raw && c.narrow) INSPIRE_LIMB_LAUNCH(4, true, kNarrowTQ, 4, qs4, o4);
+      if (raw) {
+        if (tq == 64) INSPIRE_LIMB_LAUNCH(4, true, 64, 4, qs4, o4);
+        if (tq == 48) INSPIRE_LIMB_LAUNCH(4, true, 48, 4, qs4, o4);
+        if (tq == 32) INSPIRE_LIMB_LAUNCH(4, true, 32, 4, qs4, o4);
+        if (tq == kNarrowTQ) INSPIRE_LIMB_LAUNCH(4, true, kNarrowTQ, 4, qs4, o4);
+      } else {
+        if (tq == 64) INSPIRE_LIMB_LAUNCH(4, false, 64, 4, qs4, o4);
+        if (tq == 48) INSPIRE_LIMB_LAUNCH(4, false, 48, 4, qs4, o4);
+        if (tq == 32) INSPIRE_LIMB_LAUNCH(4, false, 32, 4, qs4, o4);
+        if (tq == kNarrowTQ) INSPIRE_LIMB_LAUNCH(4, false, kNarrowTQ, 4, qs4, o4);
+      }
     } else if (nw == 7) {
       // Available(): planes, full tiles; products read mod 2^56.
       INSPIRE_LIMB_LAUNCH(8, false, 32, 7, qs8, o8);
