@@ -330,7 +330,11 @@ cudaError_t launch_typed(const void* db, int64_t db_cols, const void* q1,
           (rows + 1) / 2, db, db_cols, q1, q1_stride, pk, pk_cols, yg, yg_stride, out,
           out_stride, rows, stream);
     }
-    return launch_rows<T, DbT, MatT, 4, NQ, kThreads, false>(
+    // Three requests: prefetching segments too (32768 x 32768 u16 + 32768 x 8192
+    // i32 over Z_2^32: 590 -> 560 us). With four the second set of vectors does
+    // not fit beside the sums (635 -> 724 us), and two already run at 0.99 of
+    // the copy peak.
+    return launch_rows<T, DbT, MatT, 4, NQ, kThreads, NQ == 3>(
         (rows + 3) / 4, db, db_cols, q1, q1_stride, pk, pk_cols, yg, yg_stride, out,
         out_stride, rows, stream);
   }
