@@ -789,7 +789,8 @@ ext_step16_pair_kernel(bool first, const uint32_t* __restrict__ resid_in,
 }
 
 // Final Horner addition (or the single packed ciphertext when t == 1) and
-// the modulus switch of a to q1 and b to q2. grid = (l, batch).
+// the modulus switch of a to q1 and b to q2. grid = (l, batch, z): z blocks
+// share a ciphertext's coefficients.
 // With rescale == false it only reconstructs (component entry point).
 template <typename T>
 __global__ void __launch_bounds__(kPolyThreads)
@@ -809,8 +810,8 @@ finish_kernel(bool from_resid, const uint32_t* __restrict__ resid,
   const int64_t rbase = (static_cast<int64_t>(q) * l + shard) * c.r * 2 * d;
   T* oa = out + (static_cast<int64_t>(q) * l + shard) * 2 * d;
   T* ob = oa + d;
-#pragma unroll 4
-  for (int j = threadIdx.x; j < d; j += blockDim.x) {
+#pragma unroll 2
+  for (int j = blockIdx.z * blockDim.x + threadIdx.x; j < d; j += gridDim.z * blockDim.x) {
     T ra, rb;
     horner_state<T>(!from_resid, resid, rbase, d, j, ca, cb, c, ra, rb);
     if (rescale) {
