@@ -73,10 +73,89 @@ __device__ __forceinline__ T gadget_digit(T c, int log_modulus, int log_digit,
   return low_bits(cur, log_digit);
 }
 
-// Forward NTT of CoeffType polynomials (masked to the bits the reference's
-// chunk rule reads). grid.x = npoly * r, grid.y = batch.
+// CoeffType polynomials to transform, masked to the bits the reference's chunk
+// rule reads: of request q, `count` rows of src + q qstride + off, poly_stride
+// words apart, to dst[q][total][r][d]. Rows from `live` on are `gap` rows
+// further (an RGSW ciphertext's digits that are always zero are left out).
+template <typename T>
+struct NttRows {
+  const T* src = nullptr;
+  int64_t qstride = 0, off = 0, poly_stride = 0;
+  int count = 0, live = 0, gap = 0, total = 0;
+  T mask = 0;
+  uint32_t* dst = nullptr;
+
+  __device__ __forceinline__ int row(int i) const { return i < live ? i : i + gap; }
+  __device__ __forceinline__ const T* in(int q, int row) const {
+    return src + q * qstride + off + row * poly_stride;
+  }
+  __device__ __forceinline__ uint32_t* out(int q, int row, int r, int pi, int d) const {
+    return dst + ((static_cast<int64_t>(q) * total + row) * r + pi) * d;
+  }
+};
+
+// Forward NTTs of up to two sets of polynomials (a request's y_h and RGSW
+// rows: one launch, since at one request each is a chain of its own and two
+// of them took longer than the products they run beside).
+// grid.x = (a.count + b.count) * r, grid.y = batch.
 template <typename T, int ITERS = 0>
 __global__ void __launch_bounds__(PolyShape<ITERS>::kMaxThreads, PolyShape<ITERS>::kMinBlocks)
+ntt_rows_kernel(const NttRows<T> a, const NttRows<T> b, NttCtx c) {
+  extern __shared__ uint32_t smem[];
+  const int d = 1 << c.logd;
+  const int i = blockIdx.x / c.r;
+  const int pi = blockIdx.x % c.r;
+  const int q = blockIdx.y;
+  const bool second = i >= a.count;
+  const NttRows<T>& set = second ? b : a;
+  const int row = set.row(second ? i - a.count : i);
+  const T* in = set.in(q, row);
+  for (int j = threadIdx.x; j < d; j += blockDim.x) {
+    smem[j] = reduce_word(static_cast<T>(in[j] & set.mask), c, pi);
+  }
+  ntt_forward_t<ITERS>(smem, c, pi);
+  uint32_t* out = set.out(q, row, c.r, pi, d);
+  for (int j = threadIdx.x; j < d; j += blockDim.x) out[j] = smem[j];
+}
+
+// ntt_rows_kernel for d = 2^LOGD with the radix-16 transform of ntt16.cuh,
+// one block per polynomial over all primes (the input is read once).
+// grid = (a.count + b.count, batch), d / 16 threads, needs c.tables16.
+template <typename T, int LOGD>
+__global__ void __launch_bounds__(Ntt16<LOGD>::kThreads, 512 / Ntt16<LOGD>::kThreads)
+ntt_rows16_kernel(const NttRows<T> a, const NttRows<T> b, NttCtx c) {
+  constexpr int d = Ntt16<LOGD>::kD;
+  constexpr int NT = Ntt16<LOGD>::kThreads;
+  __shared__ uint32_t xs[d];
+  const int tid = threadIdx.x;
+  const int i = blockIdx.x;
+  const int q = blockIdx.y;
+  const bool second = i >= a.count;
+  const NttRows<T>& set = second ? b : a;
+  const int row = set.row(second ? i - a.count : i);
+  const T* in = set.in(q, row);
+  T v[16];
+#pragma unroll
+  for (int k = 0; k < 16; ++k) v[k] = in[tid + NT * k] & set.mask;
+  for (int pi = 0; pi < c.r; ++pi) {
+    const uint32_t p = c.p[pi];
+    uint32_t x[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) x[k] = reduce_word(v[k], c, pi);
+    ntt16_forward<LOGD, false, false, true>(
+        x, xs, c.tables16 + static_cast<size_t>(pi) * 2 * d, p, c.one_s[pi], tid);
+    uint4* out = reinterpret_cast<uint4*>(set.out(q, row, c.r, pi, d) + 16 * tid);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      out[w] = make_uint4(x[4 * w], x[4 * w + 1], x[4 * w + 2], x[4 * w + 3]);
+    }
+  }
+}
+
+// Forward NTT of one set of CoeffType polynomials, all rows.
+// grid.x = npoly * r, grid.y = batch.
+template <typename T>
+__global__ void __launch_bounds__(kPolyThreads)
 ntt_coeffs_kernel(const T* __restrict__ src, int64_t src_qstride,
                   int64_t src_off, int npoly, T mask, uint32_t* __restrict__ dst,
                   int64_t poly_stride, NttCtx c) {
@@ -85,48 +164,13 @@ ntt_coeffs_kernel(const T* __restrict__ src, int64_t src_qstride,
   const int poly = blockIdx.x / c.r;
   const int pi = blockIdx.x % c.r;
   const int q = blockIdx.y;
-  const uint32_t p = c.p[pi];
   const T* in = src + q * src_qstride + src_off + poly * poly_stride;
   for (int j = threadIdx.x; j < d; j += blockDim.x) {
     smem[j] = reduce_word(static_cast<T>(in[j] & mask), c, pi);
   }
-  ntt_forward_t<ITERS>(smem, c, pi);
+  ntt_forward(smem, c, pi);
   uint32_t* out = dst + ((static_cast<int64_t>(q) * npoly + poly) * c.r + pi) * d;
   for (int j = threadIdx.x; j < d; j += blockDim.x) out[j] = smem[j];
-}
-
-// ntt_coeffs_kernel for d = 2^LOGD with the radix-16 transform of ntt16.cuh,
-// one block per polynomial over all primes (the input is read once).
-// grid = (npoly, batch), d / 16 threads, needs c.tables16.
-template <typename T, int LOGD>
-__global__ void __launch_bounds__(Ntt16<LOGD>::kThreads, 512 / Ntt16<LOGD>::kThreads)
-ntt_coeffs16_kernel(const T* __restrict__ src, int64_t src_qstride,
-                    int64_t src_off, int npoly, T mask, uint32_t* __restrict__ dst,
-                    int64_t poly_stride, NttCtx c) {
-  constexpr int d = Ntt16<LOGD>::kD;
-  constexpr int NT = Ntt16<LOGD>::kThreads;
-  __shared__ uint32_t xs[d];
-  const int tid = threadIdx.x;
-  const int poly = blockIdx.x;
-  const int q = blockIdx.y;
-  const T* in = src + q * src_qstride + src_off + poly * poly_stride;
-  T v[16];
-#pragma unroll
-  for (int k = 0; k < 16; ++k) v[k] = in[tid + NT * k] & mask;
-  for (int pi = 0; pi < c.r; ++pi) {
-    const uint32_t p = c.p[pi];
-    uint32_t x[16];
-#pragma unroll
-    for (int k = 0; k < 16; ++k) x[k] = reduce_word(v[k], c, pi);
-    ntt16_forward<LOGD, false, false, true>(
-        x, xs, c.tables16 + static_cast<size_t>(pi) * 2 * d, p, c.one_s[pi], tid);
-    uint4* out = reinterpret_cast<uint4*>(
-        dst + ((static_cast<int64_t>(q) * npoly + poly) * c.r + pi) * d + 16 * tid);
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-      out[w] = make_uint4(x[4 * w], x[4 * w + 1], x[4 * w + 2], x[4 * w + 3]);
-    }
-  }
 }
 
 // Forward NTT of signed 64-bit polynomials (host-prepared operands).

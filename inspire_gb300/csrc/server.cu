@@ -696,24 +696,20 @@ PolyLaunch PolyShapeFor(int d, int64_t ctas, int sms) {
     } break;                                \
   }
 
-// Forward NTTs of npoly CoeffType polynomials per request (stride
-// poly_stride words, masked), batch requests src_qstride words apart.
+// Forward NTTs of one or two sets of a batch's polynomials.
 template <typename T>
-Status NttCoeffs(const inspire_pir_server* s, const T* src, int64_t src_qstride,
-                 int64_t src_off, int npoly, T mask, uint32_t* dst,
-                 int64_t poly_stride, const NttCtx& c, int batch, cudaStream_t st) {
+Status NttRowSets(const inspire_pir_server* s, const NttRows<T>& a, const NttRows<T>& b,
+                  const NttCtx& c, int batch, cudaStream_t st) {
   const int d = s->d;
-  if (c.tables16 != nullptr && static_cast<int64_t>(npoly) * batch >= s->sms) {
-    INSPIRE_NTT16_DISPATCH(
-        c.logd, ntt_coeffs16_kernel<T, LG><<<dim3(npoly, batch), Ntt16<LG>::kThreads, 0, st>>>(
-                    src, src_qstride, src_off, npoly, mask, dst, poly_stride, c));
+  const int count = a.count + b.count;
+  if (c.tables16 != nullptr && static_cast<int64_t>(count) * batch >= s->sms) {
+    INSPIRE_NTT16_DISPATCH(c.logd, ntt_rows16_kernel<T, LG>
+                           <<<dim3(count, batch), Ntt16<LG>::kThreads, 0, st>>>(a, b, c));
     return Cuda(cudaGetLastError(), "forward NTT");
   }
-  const PolyLaunch pl = PolyShapeFor(d, static_cast<int64_t>(npoly) * c.r * batch, s->sms);
-  dim3 grid(npoly * c.r, batch);
-  INSPIRE_ITERS_DISPATCH(pl.iters, ntt_coeffs_kernel<T, IT><<<grid, pl.nt, d * 4, st>>>(
-                                       src, src_qstride, src_off, npoly, mask, dst,
-                                       poly_stride, c));
+  const PolyLaunch pl = PolyShapeFor(d, static_cast<int64_t>(count) * c.r * batch, s->sms);
+  INSPIRE_ITERS_DISPATCH(pl.iters, ntt_rows_kernel<T, IT>
+                         <<<dim3(count * c.r, batch), pl.nt, d * 4, st>>>(a, b, c));
   return Cuda(cudaGetLastError(), "forward NTT");
 }
 
@@ -775,29 +771,65 @@ inline int64_t Ext16Min(const inspire_pir_server* s, int d) {
   return static_cast<int64_t>(s->sms) * std::max(1, 4096 / d);
 }
 
-// FinalizeMatrixPack for every shard of every request of a batch
-// (lwes_to_rlwe.cc:448-479): w->packed[q][shard] = b_agg.
 // y_h = packing_key[k..2k): forward NTT over the finalize primes.
+template <typename T>
+NttRows<T> YhRows(const inspire_pir_server* s, Workspace* w, const T* pkey) {
+  NttRows<T> n;
+  const int64_t d = s->d;
+  n.src = pkey;
+  n.qstride = 2 * s->k * d;
+  n.off = s->k * d;
+  n.poly_stride = d;
+  n.count = n.live = n.total = s->k;
+  n.mask = static_cast<T>(s->vmask_f);
+  n.dst = w->yh.get<uint32_t>();
+  return n;
+}
+
+// The RGSW b parts of the second dimension, over the eval primes; rows of
+// digits that are always zero are read by nothing.
+template <typename T>
+NttRows<T> RgswRows(const inspire_pir_server* s, Workspace* w, const T* sdim) {
+  NttRows<T> n;
+  const int64_t d = s->d;
+  n.src = sdim;
+  n.qstride = 2 * s->ne * d;
+  n.poly_stride = d;
+  n.live = LiveDigits(s->prm.log_modulus, s->prm.eval_log_digit, s->ne);
+  n.gap = s->ne - n.live;
+  n.count = 2 * n.live;
+  n.total = 2 * s->ne;
+  n.mask = static_cast<T>(s->vmask_e);
+  n.dst = w->rgswb.get<uint32_t>();
+  return n;
+}
+
 template <typename T>
 Status YhTransform(inspire_pir_server* s, Workspace* w, int batch, const T* pkey,
                    cudaStream_t st) {
-  const int d = s->d, k = s->k;
-  return NttCoeffs<T>(s, pkey, static_cast<int64_t>(2 * k) * d,
-                      static_cast<int64_t>(k) * d, k, static_cast<T>(s->vmask_f),
-                      w->yh.get<uint32_t>(), d, s->ctx_f, batch, st);
+  return NttRowSets<T>(s, YhRows(s, w, pkey), NttRows<T>{}, s->ctx_f, batch, st);
 }
 
-// The RGSW b parts of the second dimension: forward NTT over the eval
-// primes.
 template <typename T>
 Status RgswTransform(inspire_pir_server* s, Workspace* w, int batch, const T* sdim,
                      cudaStream_t st) {
-  const int d = s->d, ne = s->ne;
-  return NttCoeffs<T>(s, sdim, static_cast<int64_t>(2 * ne) * d, 0, 2 * ne,
-                      static_cast<T>(s->vmask_e), w->rgswb.get<uint32_t>(), d, s->ctx_e,
-                      batch, st);
+  return NttRowSets<T>(s, RgswRows(s, w, sdim), NttRows<T>{}, s->ctx_e, batch, st);
 }
 
+// Both, in one launch when they take the same primes.
+template <typename T>
+Status RequestTransforms(inspire_pir_server* s, Workspace* w, int batch, const T* pkey,
+                         const T* sdim, cudaStream_t st) {
+  if (s->t == 1) return YhTransform<T>(s, w, batch, pkey, st);
+  if (s->ctx_f.r == s->ctx_e.r) {
+    return NttRowSets<T>(s, YhRows(s, w, pkey), RgswRows(s, w, sdim), s->ctx_f, batch, st);
+  }
+  RETURN_IF_ERROR(YhTransform<T>(s, w, batch, pkey, st));
+  return RgswTransform<T>(s, w, batch, sdim, st);
+}
+
+// FinalizeMatrixPack for every shard of every request of a batch
+// (lwes_to_rlwe.cc:448-479): w->packed[q][shard] = b_agg.
 // yh_done: the y_h transform is already in w->yh (enqueued on another
 // stream that `st` has joined). pairs: write (a_tilde_agg, b_agg) pairs there
 // instead of the b polynomials to w->packed.
@@ -906,8 +938,7 @@ Status RunPolyStage(inspire_pir_server* s, Workspace* w, int batch,
   const int log_q = s->prm.log_modulus;
   if (s->fused_poly) {
     if (!transforms_done) {
-      RETURN_IF_ERROR(YhTransform<T>(s, w, batch, pkey, st));
-      if (t > 1) RETURN_IF_ERROR(RgswTransform<T>(s, w, batch, sdim, st));
+      RETURN_IF_ERROR(RequestTransforms<T>(s, w, batch, pkey, sdim, st));
     }
     // FinalizeMatrixPack runs inside: its time counts as polynomial
     // evaluation.
@@ -1168,19 +1199,13 @@ Status AnswerOnDevice(inspire_pir_server* s, Workspace* w, int batch,
         Cuda(cudaStreamWaitEvent(w->copy_stream, sdim_ready, 0), "wait second_dim"));
   }
   if (cb == 32) {
-    RETURN_IF_ERROR(YhTransform<uint32_t>(s, w, batch, static_cast<const uint32_t*>(pkey),
-                                          w->copy_stream));
-    if (s->t > 1) {
-      RETURN_IF_ERROR(RgswTransform<uint32_t>(
-          s, w, batch, static_cast<const uint32_t*>(sdim), w->copy_stream));
-    }
+    RETURN_IF_ERROR(RequestTransforms<uint32_t>(
+        s, w, batch, static_cast<const uint32_t*>(pkey), static_cast<const uint32_t*>(sdim),
+        w->copy_stream));
   } else {
-    RETURN_IF_ERROR(YhTransform<uint64_t>(s, w, batch, static_cast<const uint64_t*>(pkey),
-                                          w->copy_stream));
-    if (s->t > 1) {
-      RETURN_IF_ERROR(RgswTransform<uint64_t>(
-          s, w, batch, static_cast<const uint64_t*>(sdim), w->copy_stream));
-    }
+    RETURN_IF_ERROR(RequestTransforms<uint64_t>(
+        s, w, batch, static_cast<const uint64_t*>(pkey), static_cast<const uint64_t*>(sdim),
+        w->copy_stream));
   }
   RETURN_IF_ERROR(Cuda(cudaEventRecord(w->side_done, w->copy_stream), "record join"));
   if (timed) cudaEventRecord(w->ev[0], st);
@@ -1309,10 +1334,12 @@ Status ExternalOnDevice(inspire_pir_server* s, Workspace* w, int batch,
     using T = decltype(tag);
     const T* rg = static_cast<const T*>(rgsw);
     const int64_t qs = static_cast<int64_t>(2 * ng) * d;
-    RETURN_IF_ERROR(NttCoeffs<T>(s, rg, qs, 0, ng, static_cast<T>(s->vmask_e),
-                                 w->rgswa.get<uint32_t>(), 2 * d, c, batch, st));
-    RETURN_IF_ERROR(NttCoeffs<T>(s, rg, qs, d, ng, static_cast<T>(s->vmask_e),
-                                 w->rgswb.get<uint32_t>(), 2 * d, c, batch, st));
+    NttRows<T> ra = RgswRows<T>(s, w, rg), rb = ra;  // (a, b) pairs per row
+    ra.qstride = rb.qstride = qs;
+    ra.poly_stride = rb.poly_stride = 2 * d;
+    rb.off = d;
+    ra.dst = w->rgswa.get<uint32_t>();
+    RETURN_IF_ERROR(NttRowSets<T>(s, ra, rb, c, batch, st));
     ExtArgs e{s->prm.log_modulus, s->prm.eval_log_digit, ne,
               LiveDigits(s->prm.log_modulus, s->prm.eval_log_digit, ne),
               s->umask_e};
