@@ -19,7 +19,8 @@
 // for the instruction cache: one call site per transform, the prime count
 // known at compile time. With both transforms inlined at every use and the
 // general Garner reconstruction it came to 160 KB, and every phase waited on
-// instruction fetch (26 us a step at d = 4096).
+// instruction fetch (26 us a step at d = 4096; 15 us now, 30 thousand cycles:
+// transforms 10.5, products 5, inverse 6.4, barrier 1.8, words 4.5).
 //
 // G groups of d / 16 threads transform a gadget digit each (as many rounds as
 // the live digits need); then every thread takes four slots of all digits and

@@ -8,7 +8,7 @@
 // that are always zero are not read. The launches this replaces (two
 // transforms of all rows, the product, the reconstruction) wrote and read
 // every row's residues and took 152 us for 256 ciphertexts at d = 2048 over
-// Z_2^32.
+// Z_2^32 (the packing workload around them: 250 -> 183 us).
 #pragma once
 #include <cstdint>
 
