@@ -1621,14 +1621,17 @@ Status CreateServer(const inspire_pir_params* prm, const void* db,
         s->k + (t > 1 ? 2 * LiveDigits(prm->log_modulus, prm->eval_log_digit, s->ne) : 0);
     if (PrimesFor(bits, &need, set).ok() && need <= r && terms <= 30) {
       s->fused_poly = true;
-      r_f = r_e = r;
+      r_f = r;
+      // A server without EvalPoly still multiplies by RGSW ciphertexts, whose
+      // products may need more primes than its answers.
+      if (t > 1) r_e = r;
     }
   }
-  // The server's calls come on streams of their own: wait for the tables.
   if (set == kSet27 && d <= 4096 && se.ok()) {
     s->fused_ext =
         r_e <= (cb == 32 ? AnswerPolyPrimes<uint32_t>() : AnswerPolyPrimes<uint64_t>());
   }
+  // The server's calls come on streams of their own: wait for the tables.
   RETURN_IF_ERROR(NttTables::Create(prm->log_degree, set, nullptr, &s->tables, false));
   RETURN_IF_ERROR(Cuda(cudaStreamSynchronize(nullptr), "NTT tables"));
   {

@@ -50,3 +50,10 @@ def test_matches_oracle(d, bits, log_q, evalg, batch):
                                       rgsw[i].reshape(-1, d))
         assert np.array_equal(got[i, 0], wa), i
         assert np.array_equal(got[i, 1], wb), i
+
+
+@pytest.mark.parametrize("evalg", [(40, 1), (32, 2)])
+def test_one_slice_server_with_wide_digits(evalg):
+    # Products of 116 and 109 bits: five 27-bit primes, where the answers of
+    # the same server take four.
+    test_matches_oracle(2048, 64, 64, evalg, 2)
