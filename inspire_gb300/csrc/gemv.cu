@@ -324,8 +324,24 @@ cudaError_t launch_typed(const void* db, int64_t db_cols, const void* q1,
     // matrix at NQ = 4, so three or four queries take four rows too (4 queries
     // at 32768 x 32768 u16 + 32768 x 8192 i32 over Z_2^32: 728 -> 635 us).
     // Below 8192 rows the blocks would fill the device barely twice and two
-    // rows stay ahead (4096 rows over Z_2^64: 58 against 62 us).
-    if (NQ >= 3 && rows < 8192) {
+    // rows stay ahead (4096 rows over Z_2^64: 58 against 62 us), except for
+    // three queries and a u8 database, whose 16 words a query per vector make
+    // the loads the bound at any size.
+    const bool few = rows < 8192 && !(NQ == 3 && sizeof(DbT) == 1);
+    // The pack segment's vectors hold four words or two, so there the sums of
+    // four rows by four queries cost more than the shared loads give: over
+    // Z_2^64 with a u16 database, and over Z_2^32 with a u8 one, four rows need
+    // as many bytes of database as of pack matrix, or a quarter (us with two
+    // and four rows of four queries, database : pack in MB: Z_2^64, u16 + i32,
+    // 537 : 268 607, 523; 537 : 537 688, 673; 537 : 1074 898, 954; Z_2^32, u8 +
+    // i32, 268 : 1074 528, 517; 67 : 1074 365, 393). The other types gain at
+    // any share.
+    const int64_t db_bytes = db_cols * static_cast<int64_t>(sizeof(DbT));
+    const int64_t pk_bytes = pk_cols * static_cast<int64_t>(sizeof(MatT));
+    const bool pack_bound =
+        NQ == 4 && ((sizeof(T) == 8 && sizeof(DbT) == 2 && pk_bytes > db_bytes) ||
+                    (sizeof(T) == 4 && sizeof(DbT) == 1 && pk_bytes > 4 * db_bytes));
+    if (NQ >= 3 && (few || pack_bound)) {
       return launch_rows<T, DbT, MatT, 2, NQ, kThreads, false>(
           (rows + 1) / 2, db, db_cols, q1, q1_stride, pk, pk_cols, yg, yg_stride, out,
           out_stride, rows, stream);
