@@ -481,12 +481,12 @@ hint_rows_kernel(const S* __restrict__ db, int64_t cols, int n,
 }
 
 // v[0] = a[0], v[j] = -a[d - j] for each a-component
-// (hint_computation.cc:110-119). grid = (ceil(d / 256), n).
+// (hint_computation.cc:110-119). grid = (n, ceil(d / 256)).
 template <typename T>
 __global__ void invert_components_kernel(const T* __restrict__ a, int d, T* __restrict__ v) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  const int j = blockIdx.y * blockDim.x + threadIdx.x;
   if (j >= d) return;
-  const int64_t k = static_cast<int64_t>(blockIdx.y) * d;
+  const int64_t k = static_cast<int64_t>(blockIdx.x) * d;
   v[k + j] = j == 0 ? a[k] : static_cast<T>(T{0} - a[k + d - j]);
 }
 

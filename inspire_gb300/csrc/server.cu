@@ -3620,7 +3620,7 @@ int inspire_compute_hint_matrix(int32_t db_kind, int32_t coeff_bits, const void*
                 static_cast<T*>(out_dev), c, crt));
         return Cuda(cudaGetLastError(), "hint rows");
       }
-      invert_components_kernel<T><<<dim3((d + 255) / 256, n), 256, 0, cs>>>(a, d, dres.get<T>());
+      invert_components_kernel<T><<<dim3(n, (d + 255) / 256), 256, 0, cs>>>(a, d, dres.get<T>());
       RETURN_IF_ERROR(Cuda(cudaGetLastError(), "a-component inversion"));
       ntt_coeffs_kernel<T><<<dim3(n * r, 1), PolyThreads(d), d * 4, cs>>>(
           dres.get<T>(), 0, 0, n, static_cast<T>(~0ull), dV.get<uint32_t>(), d, c);

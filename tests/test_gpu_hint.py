@@ -100,3 +100,32 @@ def test_hint_device_pointers_match_host_call():
     assert rc == 0, err.value
     torch.cuda.synchronize()
     assert np.array_equal(t_out.cpu().numpy().view(np.uint32), want)
+
+
+@pytest.mark.parametrize("tdt", [np.uint32, np.uint64])
+@pytest.mark.parametrize("d", [2, 512])
+def test_more_components_than_a_grid_dimension_holds(d, tdt):
+    # n above 65535; the hint is linear in the database, so single entries
+    # and their sum are checked against rotated components.
+    n = 65537
+    rng = np.random.default_rng(d)
+    a = rng.integers(0, np.iinfo(tdt).max, size=(n, d), dtype=tdt,
+                     endpoint=True)
+    db = np.zeros((3, n * d), dtype=np.uint8)
+    db[0, (n - 1) * d] = 3
+    db[1, 65535 * d + 1] = 255
+    db[2, 7 * d] = 1
+    db[2, (n - 1) * d + 1] = 2
+    got = pir.ComputeHintMatrix(db, a)
+
+    def times_x(v):  # row k = 1 of M_b: out[j] = a[1 - j], negated beyond
+        return np.concatenate([v[1:2], v[0:1], (0 - v[:1:-1]).astype(tdt)])[:d]
+
+    def inverted(v):
+        return np.concatenate([v[:1], (0 - v[:0:-1]).astype(tdt)])
+
+    with np.errstate(over="ignore"):
+        assert np.array_equal(got[0], (inverted(a[n - 1]) * tdt(3)).astype(tdt))
+        assert np.array_equal(got[1], (times_x(a[65535]) * tdt(255)).astype(tdt))
+        assert np.array_equal(got[2], (inverted(a[7])
+                                       + times_x(a[n - 1]) * tdt(2)).astype(tdt))
