@@ -377,14 +377,17 @@ pp_tail_kernel(const T* __restrict__ fin, ChainArgs a, NttCtx c, T* __restrict__
 // primes g, g + G, ..., each group's transforms synchronising on named
 // barrier g + 1, so the k forward transforms and the inverse of G primes run
 // side by side; the residues meet in shared memory (res, natural
-// coefficient order) for the CRT. xs: G exchange buffers of d words; dig:
-// the k digit planes of `cur` (k d words of T). The link is a chain of
+// coefficient order) for the CRT, each prime's d words serving its transforms
+// as the exchange buffer before they take its residues (apart, the buffers of
+// G groups kept three digits at d = 4096 and ten at d = 2048 over Z_2^64 out of
+// this form: 259 and 218 ms for a slice on pp_chain_kernel). dig: the k digit
+// planes of `cur` (k d words of T). The link is a chain of
 // dependent steps, so the digit planes go to shared memory for the
 // transforms (and out to `digits` for the matrix, not read back), and
 // `add` is loaded while other groups finish. Signed digits of up to
 // 27 bits are below p, so their residues need no division. Same words as pp_link.
 template <typename T, int LOGD, int G>
-__device__ __forceinline__ void pp_link16(T* cur, uint32_t* res, uint32_t* xs, T* dig,
+__device__ __forceinline__ void pp_link16(T* cur, uint32_t* res, T* dig,
                                           const ChainArgs& a, const NttCtx& c, int power,
                                           const uint32_t* W, T* digits, const T* add) {
   using S = typename std::make_signed<T>::type;
@@ -402,8 +405,8 @@ __device__ __forceinline__ void pp_link16(T* cur, uint32_t* res, uint32_t* xs, T
     for (int l = 0; l < a.k; ++l) digits[static_cast<int64_t>(l) * d + r] = dig[l * d + r];
   }
   __syncthreads();
-  uint32_t* x_buf = xs + g * d;
   for (int pi = g; pi < c.r; pi += G) {
+    uint32_t* x_buf = res + static_cast<int64_t>(pi) * d;
     const uint32_t p = c.p[pi];
     const uint32_t pinv = c.pinv[pi];
     const uint2* tab16 = c.tables16 + static_cast<size_t>(pi) * 2 * d;
@@ -467,8 +470,7 @@ __device__ __forceinline__ void pp_link16(T* cur, uint32_t* res, uint32_t* xs, T
 }
 
 // pp_chain_kernel with pp_link16: grid = (2, slices), block = G d/16
-// threads, shared memory (1 + k) d words of T + (r + G) d words (needs
-// c.tables16).
+// threads, shared memory (1 + k) d words of T + r d words (needs c.tables16).
 template <typename T, int LOGD, int G>
 __global__ void __launch_bounds__(G * Ntt16<LOGD>::kThreads, 1)
 pp_chain16_kernel(const T* __restrict__ ev, ChainArgs a, NttCtx c, T* __restrict__ tg,
@@ -477,8 +479,7 @@ pp_chain16_kernel(const T* __restrict__ ev, ChainArgs a, NttCtx c, T* __restrict
   constexpr int d = 1 << LOGD;
   T* cur = reinterpret_cast<T*>(pp_smem);
   uint32_t* res = reinterpret_cast<uint32_t*>(cur + d);
-  uint32_t* xs = res + static_cast<int64_t>(c.r) * d;
-  T* dig = reinterpret_cast<T*>(xs + G * d);
+  T* dig = reinterpret_cast<T*>(res + static_cast<int64_t>(c.r) * d);
   const int chain = blockIdx.x, s = blockIdx.y;
   const T* evs = ev + static_cast<int64_t>(s) * d * d;
   const T* start = evs + static_cast<int64_t>(__ldg(a.hat_row + (chain == 0 ? d / 2 - 1 : d - 1))) * d;
@@ -491,7 +492,7 @@ pp_chain16_kernel(const T* __restrict__ ev, ChainArgs a, NttCtx c, T* __restrict
                           ? p5
                           : static_cast<int>((static_cast<int64_t>(p5) * (2 * d - 1)) % (2 * d));
     const T* add = evs + static_cast<int64_t>(__ldg(a.hat_row + (chain == 0 ? i : d / 2 + i))) * d;
-    pp_link16<T, LOGD, G>(cur, res, xs, dig, a, c, power, a.Wg,
+    pp_link16<T, LOGD, G>(cur, res, dig, a, c, power, a.Wg,
                           out + static_cast<int64_t>(i) * a.k * d, add);
   }
   T* f = fin + (static_cast<int64_t>(s) * 2 + chain) * d;
@@ -507,14 +508,13 @@ pp_tail16_kernel(const T* __restrict__ fin, ChainArgs a, NttCtx c, T* __restrict
   constexpr int d = 1 << LOGD;
   T* cur = reinterpret_cast<T*>(pp_smem);
   uint32_t* res = reinterpret_cast<uint32_t*>(cur + d);
-  uint32_t* xs = res + static_cast<int64_t>(c.r) * d;
-  T* dig = reinterpret_cast<T*>(xs + G * d);
+  T* dig = reinterpret_cast<T*>(res + static_cast<int64_t>(c.r) * d);
   const int s = blockIdx.x;
   const T* tgf = fin + static_cast<int64_t>(s) * 2 * d;
   const T* tghf = tgf + d;
   for (int r = threadIdx.x; r < d; r += blockDim.x) cur[r] = tghf[r];
   __syncthreads();
-  pp_link16<T, LOGD, G>(cur, res, xs, dig, a, c, 1, a.Wh,
+  pp_link16<T, LOGD, G>(cur, res, dig, a, c, 1, a.Wh,
                         t_vec_h + static_cast<int64_t>(s) * a.k * d, tgf);
   for (int r = threadIdx.x; r < d; r += blockDim.x) {
     a_tilde[static_cast<int64_t>(s) * d + r] = pp_low<T>(cur[r], a.log_q);

@@ -3922,10 +3922,10 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
     // The radix-16 register transforms (d = 2048..8192): G groups of d/16
     // threads, one prime each at a time, at most 768 threads (85 registers
     // a thread).
+    const size_t smem16 = (1 + k) * d * w + static_cast<size_t>(d) * 4 * r;
     auto chains16 = [&](auto ltag, auto gtag) -> Status {
       constexpr int LG = decltype(ltag)::value;
       constexpr int GR = decltype(gtag)::value;
-      const size_t smem16 = (1 + k) * d * w + static_cast<size_t>(d) * 4 * (r + GR);
       RETURN_IF_ERROR(SetSmem(pp_chain16_kernel<T, LG, GR>, smem16));
       RETURN_IF_ERROR(SetSmem(pp_tail16_kernel<T, LG, GR>, smem16));
       constexpr int nt = GR * Ntt16<LG>::kThreads;
@@ -3959,7 +3959,6 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
                                               dtg.get<T>(), dtgh.get<T>(), dfin.get<T>()),
                            "reduction chains"));
       constexpr int GT = LG == 11 ? 3 : 2;
-      const size_t smem16 = (1 + k) * d * w + static_cast<size_t>(d) * 4 * (r + GT);
       RETURN_IF_ERROR(SetSmem(pp_tail16_kernel<T, LG, GT>, smem16));
       pp_tail16_kernel<T, LG, GT><<<slices, GT * Ntt16<LG>::kThreads, smem16, cs>>>(
           dfin.get<T>(), ca, c, static_cast<T*>(th_out), static_cast<T*>(a_out));
@@ -3971,8 +3970,7 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
     using I4 = std::integral_constant<int, 4>;
     using I5 = std::integral_constant<int, 5>;
     const int groups16 = logd == 11 ? std::min(r, 5) : logd == 12 ? std::min(r, 3) : 1;
-    const bool fits16 =
-        (1 + k) * d * w + static_cast<size_t>(d) * 4 * (r + groups16) <= 227 * 1024;
+    const bool fits16 = smem16 <= 227 * 1024;
     if (clusters && fits16) {
       if (logd == 11) {
         RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 11>{}));
