@@ -3777,9 +3777,10 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
     return fail("null buffer.");
   }
   const int k = num_digits;
+  const size_t w = coeff_bits / 8;
   int r = 0;
   const double bits = BoundBits(k, d, log_digit, coeff_bits);
-  const PrimeSet set = SetFor(logd, bits);
+  PrimeSet set = SetFor(logd, bits);
   Status st = PrimesFor(bits, &r, set);
   if (!st.ok()) return Report(st, err, err_len);
   // d = 2048 and 4096: a cluster per chain (chain16.cuh), with as many primes
@@ -3790,9 +3791,21 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
   const bool clusters = set == kSet27 && r <= chain_r && log_digit <= 27 && k <= 30 &&
                         cluster_smem <= 227 * 1024;
   if (clusters) r = chain_r;
+  // The radix-16 links (pp_link16) keep the digits and the residues in shared
+  // memory. Rings that do not fit run the general ones, whose time and shared
+  // memory go with the number of primes and which 27-bit primes do not speed
+  // up: the 31-bit set, which holds a product in as many or fewer (digits of
+  // 10 bits, k = 5, over Z_2^64: three instead of four, 305 against 402 ms a
+  // slice at d = 4096).
+  const size_t smem16 = (1 + k) * d * w + static_cast<size_t>(d) * 4 * r;
+  const bool fits16 = set == kSet27 && smem16 <= 227 * 1024;
+  if (!fits16) {
+    set = kSet31;
+    st = PrimesFor(bits, &r, set);
+    if (!st.ok()) return Report(st, err, err_len);
+  }
   const int iters = d > 4096 ? 2 : 1;
   const int threads = d / (4 * iters);
-  const size_t w = coeff_bits / 8;
   const size_t chain_smem = d * w + static_cast<size_t>(d) * 4 * (1 + r);
   if (chain_smem > 227 * 1024) return fail("ring degree and gadget too large.");
   const cudaStream_t cs = on_device ? static_cast<cudaStream_t>(stream) : nullptr;
@@ -3922,7 +3935,6 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
     // The radix-16 register transforms (d = 2048..8192): G groups of d/16
     // threads, one prime each at a time, at most 768 threads (85 registers
     // a thread).
-    const size_t smem16 = (1 + k) * d * w + static_cast<size_t>(d) * 4 * r;
     auto chains16 = [&](auto ltag, auto gtag) -> Status {
       constexpr int LG = decltype(ltag)::value;
       constexpr int GR = decltype(gtag)::value;
@@ -3970,22 +3982,21 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
     using I4 = std::integral_constant<int, 4>;
     using I5 = std::integral_constant<int, 5>;
     const int groups16 = logd == 11 ? std::min(r, 5) : logd == 12 ? std::min(r, 3) : 1;
-    const bool fits16 = smem16 <= 227 * 1024;
     if (clusters && fits16) {
       if (logd == 11) {
         RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 11>{}));
       } else {
         RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 12>{}));
       }
-    } else if (c.tables16 != nullptr && fits16 && logd == 11) {
+    } else if (fits16 && logd == 11) {
       if (groups16 == 2) RETURN_IF_ERROR(chains16(std::integral_constant<int, 11>{}, I2{}));
       if (groups16 == 3) RETURN_IF_ERROR(chains16(std::integral_constant<int, 11>{}, I3{}));
       if (groups16 == 4) RETURN_IF_ERROR(chains16(std::integral_constant<int, 11>{}, I4{}));
       if (groups16 == 5) RETURN_IF_ERROR(chains16(std::integral_constant<int, 11>{}, I5{}));
-    } else if (c.tables16 != nullptr && fits16 && logd == 12) {
+    } else if (fits16 && logd == 12) {
       if (groups16 == 2) RETURN_IF_ERROR(chains16(std::integral_constant<int, 12>{}, I2{}));
       if (groups16 == 3) RETURN_IF_ERROR(chains16(std::integral_constant<int, 12>{}, I3{}));
-    } else if (c.tables16 != nullptr && fits16 && logd == 13) {
+    } else if (fits16 && logd == 13) {
       RETURN_IF_ERROR(chains16(std::integral_constant<int, 13>{}, I1{}));
     } else if (iters == 2) {
       RETURN_IF_ERROR(chains(std::integral_constant<int, 2>{}));

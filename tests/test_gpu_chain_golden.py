@@ -39,3 +39,10 @@ def test_digest_sees_one_word():
     y = x.copy()
     y[3] ^= np.uint64(1)
     assert chains.digest(x) != chains.digest(y)
+
+
+@pytest.mark.parametrize("name", ["d8192_u64_q64_30x1"])
+def test_general_chains_of_wide_rings(name):
+    # Digits of 29 bits and more over Z_2^64: four 31-bit primes fit, five
+    # 27-bit ones do not.
+    check(name)
