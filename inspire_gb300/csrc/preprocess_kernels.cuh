@@ -385,7 +385,9 @@ pp_tail_kernel(const T* __restrict__ fin, ChainArgs a, NttCtx c, T* __restrict__
 // dependent steps, so the digit planes go to shared memory for the
 // transforms (and out to `digits` for the matrix, not read back), and
 // `add` is loaded while other groups finish. Signed digits of up to
-// 27 bits are below p, so their residues need no division. Same words as pp_link.
+// 27 bits are below p; wider ones are reduced with the primes' Shoup constants
+// (with a 64-bit remainder for each, digits of 28 bits over Z_2^64 took 36
+// ms a slice at d = 2048). Same words as pp_link.
 template <typename T, int LOGD, int G>
 __device__ __forceinline__ void pp_link16(T* cur, uint32_t* res, T* dig,
                                           const ChainArgs& a, const NttCtx& c, int power,
@@ -424,7 +426,9 @@ __device__ __forceinline__ void pp_link16(T* cur, uint32_t* res, T* dig,
           x[q] = v < 0 ? static_cast<uint32_t>(static_cast<int64_t>(v) + p)
                        : static_cast<uint32_t>(v);
         } else {
-          x[q] = pp_signed_residue(static_cast<int64_t>(v), p);
+          const T u = static_cast<T>(v);
+          const uint32_t m = reduce_word(v < 0 ? static_cast<T>(T{0} - u) : u, c, pi);
+          x[q] = v < 0 ? p - m : m;
         }
       }
       ntt16_forward<LOGD, false, kCompact>(x, x_buf, tab16, p, c.one_s[pi], lt, g + 1);
