@@ -19,25 +19,29 @@
 
 namespace inspire {
 
-// Digits transformed side by side; blocks of G groups of d / 16 threads (the
-// other groups help with the products and the reconstruction).
+// Digits transformed side by side at most; blocks of G groups of d / 16 threads
+// (the other groups help with the products and the reconstruction).
 constexpr int kChainSide = 2;
 
-// Bytes of shared memory: twiddle pairs, key-part transforms, exchange
-// buffers, residues, digit planes.
+// Bytes of shared memory with `side` digits side by side: twiddle pairs,
+// key-part transforms, exchange buffers, residues, digit planes. Two where
+// they fit (up to three digits at d = 4096, ten at d = 2048), else one: a
+// block per chain takes longer by more (four digits at d = 4096 over Z_2^32:
+// 83 ms a slice).
 template <int LOGD>
-constexpr size_t Chain16Smem(int k) {
-  return static_cast<size_t>(Ntt16<LOGD>::kD) * 4 * (4 + k + kChainSide + 1 + k);
+constexpr size_t Chain16Smem(int k, int side) {
+  return static_cast<size_t>(Ntt16<LOGD>::kD) * 4 * (4 + k + side + 1 + k);
 }
 
 #ifdef __CUDACC__
-// grid = (2 R, slices), clusters of R, G d / 16 threads. Needs log_digit <= 27
+// grid = (2 R, slices), clusters of R, G d / 16 threads, side digits side by
+// side (Chain16Smem). Needs log_digit <= 27
 // and at most 30 digits. Outputs as pp_chain_kernel's.
 template <typename T, int LOGD, int G, int R>
 __global__ void __launch_bounds__(G * Ntt16<LOGD>::kThreads, 1)
 chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainArgs a,
                        const __grid_constant__ NttCtx c, const __grid_constant__ CrtArgs crt,
-                       T* __restrict__ tg, T* __restrict__ tgh, T* __restrict__ fin) {
+                       int side, T* __restrict__ tg, T* __restrict__ tgh, T* __restrict__ fin) {
   extern __shared__ __align__(16) uint32_t smem[];
   constexpr int d = Ntt16<LOGD>::kD;
   constexpr int NT = Ntt16<LOGD>::kThreads;
@@ -58,9 +62,9 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
   const uint2* tw = reinterpret_cast<const uint2*>(smem);
   const uint2* itw = tw + d;
   uint32_t* W = smem + 4 * d;                              // [k][d]
-  uint32_t* regions = W + static_cast<int64_t>(k) * d;     // [kChainSide][d]
+  uint32_t* regions = W + static_cast<int64_t>(k) * d;     // [side][d]
   uint32_t* region = regions + grp * d;
-  uint32_t* res = regions + kChainSide * d;
+  uint32_t* res = regions + side * d;
   int32_t* dig = reinterpret_cast<int32_t*>(res + d);      // [k][d]
   {
     const uint4* src =
@@ -128,8 +132,8 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
     }
     uint32_t x[16];
 #pragma unroll 1
-    for (int l0 = 0; l0 < k; l0 += kChainSide) {
-      if (grp < kChainSide && l0 + grp < k) {
+    for (int l0 = 0; l0 < k; l0 += side) {
+      if (grp < side && l0 + grp < k) {
         const int32_t* src = dig + (l0 + grp) * d + lt;
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
@@ -153,14 +157,14 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
             const int at = ntt16_pos<LOGD>(e + m);
 #pragma unroll
             for (int o = 0; o < kChainSide; ++o) {
-              if (l0 + o < k) {
+              if (o < side && l0 + o < k) {
                 sum[u][m] += static_cast<uint64_t>(regions[o * d + at]) * W[(l0 + o) * d + from];
               }
             }
           }
         }
       }
-      if (l0 + kChainSide < k) __syncthreads();
+      if (l0 + side < k) __syncthreads();
     }
 #pragma unroll
     for (int u = 0; u < kQuads; ++u) {

@@ -3786,8 +3786,12 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
   // d = 2048 and 4096: a cluster per chain (chain16.cuh), with as many primes
   // as its code is built for.
   const int chain_r = coeff_bits == 32 ? AnswerPolyPrimes<uint32_t>() : AnswerPolyPrimes<uint64_t>();
-  const size_t cluster_smem =
-      logd == 11 ? Chain16Smem<11>(k) : logd == 12 ? Chain16Smem<12>(k) : SIZE_MAX;
+  auto chain16_smem = [&](int side) {
+    return logd == 11 ? Chain16Smem<11>(k, side)
+                      : logd == 12 ? Chain16Smem<12>(k, side) : SIZE_MAX;
+  };
+  const int chain_side = chain16_smem(kChainSide) <= 227 * 1024 ? kChainSide : 1;
+  const size_t cluster_smem = chain16_smem(chain_side);
   const bool clusters = set == kSet27 && r <= chain_r && log_digit <= 27 && k <= 30 &&
                         cluster_smem <= 227 * 1024;
   if (clusters) r = chain_r;
@@ -3967,7 +3971,7 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
       cfg.attrs = &cluster;
       cfg.numAttrs = 1;
       const CrtArgs crt = tabs->Crt(R);
-      RETURN_IF_ERROR(Cuda(cudaLaunchKernelEx(&cfg, kernel, ev->get<T>(), ca, c, crt,
+      RETURN_IF_ERROR(Cuda(cudaLaunchKernelEx(&cfg, kernel, ev->get<T>(), ca, c, crt, chain_side,
                                               dtg.get<T>(), dtgh.get<T>(), dfin.get<T>()),
                            "reduction chains"));
       constexpr int GT = LG == 11 ? 3 : 2;
