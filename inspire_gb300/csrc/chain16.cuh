@@ -1,5 +1,6 @@
 // The reduction chains of PreprocessPack (crypto/lwes_to_rlwe.cc:310-344) for
-// d = 2048 and 4096, a cluster of one CTA per prime for each (chain, slice).
+// d = 2048 and 4096, and d = 8192 over Z_2^32, a cluster of one CTA per prime
+// for each (chain, slice).
 //
 // A chain is d/2 - 1 dependent links: signed digits of the running word
 // vector, their products with the key parts read through an automorphism, an
@@ -10,7 +11,8 @@
 // through distributed shared memory, and the code is one transform body each
 // way. The one-block form (all primes side by side, twiddles and permuted key
 // words from L2, 75 KB of code) took 20 us a link at d = 2048 over Z_2^64, this
-// one 5.5 (chains of 8 slices 23.7 -> 5.65 ms).
+// one 5.5 (chains of 8 slices 23.7 -> 5.65 ms). At d = 8192 twiddles and key-part
+// transforms do not fit beside the rest and stay in L2.
 #pragma once
 #include <cstdint>
 
@@ -30,7 +32,8 @@ constexpr int kChainSide = 2;
 // 83 ms a slice).
 template <int LOGD>
 constexpr size_t Chain16Smem(int k, int side) {
-  return static_cast<size_t>(Ntt16<LOGD>::kD) * 4 * (4 + k + side + 1 + k);
+  return static_cast<size_t>(Ntt16<LOGD>::kD) * 4 *
+         ((LOGD <= 12 ? 4 + k : 0) + side + 1 + k);
 }
 
 #ifdef __CUDACC__
@@ -48,6 +51,7 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
   constexpr int kThreads = G * NT;
   constexpr int kQuads = (d / 4 + kThreads - 1) / kThreads;
   constexpr int kWords = (d + kThreads - 1) / kThreads;
+  constexpr bool kLocal = LOGD <= 12;  // twiddles and key parts in shared memory
   static_assert(G >= kChainSide, "a group per digit");
   using S = typename std::make_signed<T>::type;
   const int tid = threadIdx.x;
@@ -59,19 +63,20 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
   const int s = blockIdx.y;
   const int k = a.k;
   const uint32_t p = c.p[pi], pinv = c.pinv[pi], one_s = c.one_s[pi];
-  const uint2* tw = reinterpret_cast<const uint2*>(smem);
+  const uint2* tables = c.tables16 + static_cast<size_t>(pi) * 2 * d;
+  const uint2* tw = kLocal ? reinterpret_cast<const uint2*>(smem) : tables;
   const uint2* itw = tw + d;
-  uint32_t* W = smem + 4 * d;                              // [k][d]
-  uint32_t* regions = W + static_cast<int64_t>(k) * d;     // [side][d]
+  const int w_stride = kLocal ? d : R * d;
+  const uint32_t* W = kLocal ? smem + 4 * d : a.Wg + pi * d;        // [k][w_stride]
+  uint32_t* regions = smem + (kLocal ? (4 + k) * d : 0);            // [side][d]
   uint32_t* region = regions + grp * d;
   uint32_t* res = regions + side * d;
   int32_t* dig = reinterpret_cast<int32_t*>(res + d);      // [k][d]
-  {
-    const uint4* src =
-        reinterpret_cast<const uint4*>(c.tables16 + static_cast<size_t>(pi) * 2 * d);
+  if constexpr (kLocal) {
+    const uint4* src = reinterpret_cast<const uint4*>(tables);
     uint4* dst = reinterpret_cast<uint4*>(smem);
     for (int i = tid; i < d; i += kThreads) dst[i] = __ldg(src + i);
-    uint4* wd = reinterpret_cast<uint4*>(W);
+    uint4* wd = reinterpret_cast<uint4*>(smem + 4 * d);
     for (int i = tid; i < k * (d / 4); i += kThreads) {
       const int l = i / (d / 4);
       wd[i] = __ldg(reinterpret_cast<const uint4*>(
@@ -140,7 +145,7 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
           const int32_t v = src[NT * m];
           x[m] = static_cast<uint32_t>(v) + (v < 0 ? p : 0u);
         }
-        ntt16_forward<LOGD, true>(x, region, tw, p, one_s, lt, bar);
+        ntt16_forward<LOGD, kLocal, !kLocal>(x, region, tw, p, one_s, lt, bar);
         ntt16_store_slots<LOGD>(x, region, lt);
       }
       __syncthreads();
@@ -158,7 +163,9 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
 #pragma unroll
             for (int o = 0; o < kChainSide; ++o) {
               if (o < side && l0 + o < k) {
-                sum[u][m] += static_cast<uint64_t>(regions[o * d + at]) * W[(l0 + o) * d + from];
+                const uint32_t* w = W + (l0 + o) * w_stride + from;
+                sum[u][m] += static_cast<uint64_t>(regions[o * d + at]) *
+                             (kLocal ? *w : __ldg(w));
               }
             }
           }
@@ -180,7 +187,7 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
     __syncthreads();
     if (grp == 0) {
       ntt16_load_slots<LOGD>(x, region, lt);
-      ntt16_inverse<LOGD, true>(x, region, itw, p, one_s, lt, bar);
+      ntt16_inverse<LOGD, kLocal, !kLocal>(x, region, itw, p, one_s, lt, bar);
 #pragma unroll
       for (int m = 0; m < 16; ++m) {
         res[lt + NT * m] = shoup_mul(x[m], crt.scale[pi], crt.scale_s[pi], p);

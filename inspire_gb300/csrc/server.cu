@@ -3783,12 +3783,14 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
   PrimeSet set = SetFor(logd, bits);
   Status st = PrimesFor(bits, &r, set);
   if (!st.ok()) return Report(st, err, err_len);
-  // d = 2048 and 4096: a cluster per chain (chain16.cuh), with as many primes
-  // as its code is built for.
+  // d = 2048 and 4096, and d = 8192 over Z_2^32: a cluster per chain
+  // (chain16.cuh), with as many primes as its code is built for.
   const int chain_r = coeff_bits == 32 ? AnswerPolyPrimes<uint32_t>() : AnswerPolyPrimes<uint64_t>();
   auto chain16_smem = [&](int side) {
-    return logd == 11 ? Chain16Smem<11>(k, side)
-                      : logd == 12 ? Chain16Smem<12>(k, side) : SIZE_MAX;
+    return logd == 11   ? Chain16Smem<11>(k, side)
+           : logd == 12 ? Chain16Smem<12>(k, side)
+           : logd == 13 && coeff_bits == 32 ? Chain16Smem<13>(k, side)
+                                            : SIZE_MAX;
   };
   const int chain_side = chain16_smem(kChainSide) <= 227 * 1024 ? kChainSide : 1;
   const size_t cluster_smem = chain16_smem(chain_side);
@@ -3954,7 +3956,7 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
     };
     auto chain_clusters = [&](auto ltag) -> Status {
       constexpr int LG = decltype(ltag)::value;
-      constexpr int GR = 4;
+      constexpr int GR = LG <= 12 ? 4 : 2;
       constexpr int R = AnswerPolyPrimes<T>();
       auto* kernel = chain16_cluster_kernel<T, LG, GR, R>;
       RETURN_IF_ERROR(SetSmem(kernel, cluster_smem));
@@ -3974,7 +3976,7 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
       RETURN_IF_ERROR(Cuda(cudaLaunchKernelEx(&cfg, kernel, ev->get<T>(), ca, c, crt, chain_side,
                                               dtg.get<T>(), dtgh.get<T>(), dfin.get<T>()),
                            "reduction chains"));
-      constexpr int GT = LG == 11 ? 3 : 2;
+      constexpr int GT = LG == 11 ? 3 : LG == 12 ? 2 : 1;
       RETURN_IF_ERROR(SetSmem(pp_tail16_kernel<T, LG, GT>, smem16));
       pp_tail16_kernel<T, LG, GT><<<slices, GT * Ntt16<LG>::kThreads, smem16, cs>>>(
           dfin.get<T>(), ca, c, static_cast<T*>(th_out), static_cast<T*>(a_out));
@@ -3989,8 +3991,10 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
     if (clusters && fits16) {
       if (logd == 11) {
         RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 11>{}));
-      } else {
+      } else if (logd == 12) {
         RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 12>{}));
+      } else if constexpr (sizeof(T) == 4) {
+        RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 13>{}));
       }
     } else if (fits16 && logd == 11) {
       if (groups16 == 2) RETURN_IF_ERROR(chains16(std::integral_constant<int, 11>{}, I2{}));

@@ -46,3 +46,9 @@ def test_general_chains_of_wide_rings(name):
     # Digits of 29 bits and more over Z_2^64: four 31-bit primes fit, five
     # 27-bit ones do not.
     check(name)
+
+
+@pytest.mark.parametrize("name", ["d8192_u32_q32_12x2"])
+def test_cluster_chains_at_d8192(name):
+    # Twiddles and key parts from global memory.
+    check(name)
