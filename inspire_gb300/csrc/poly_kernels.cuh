@@ -638,8 +638,10 @@ ext_step_kernel(bool first, const uint32_t* __restrict__ resid_in,
 // passes of ntt16.cuh, the RGSW products are taken in the layout the forward
 // transform leaves (16 consecutive slots per thread, 16-byte loads) and the
 // inverse starts from the accumulators without a trip through shared
-// memory. Same residues as ext_step_kernel. grid = (l, batch), d / 16 threads,
-// needs c.tables16.
+// memory. With gridDim.z blocks per (shard, request) block z takes the primes
+// z, z + gridDim.z, ... (each reconstructs the state for itself). Same
+// residues as ext_step_kernel. grid = (l, batch, 1..r), d / 16 threads, needs
+// c.tables16.
 template <typename T, int LOGD>
 __global__ void __launch_bounds__(Ntt16<LOGD>::kThreads, 512 / Ntt16<LOGD>::kThreads)
 ext_step16_kernel(bool first, const uint32_t* __restrict__ resid_in,
@@ -671,7 +673,7 @@ ext_step16_kernel(bool first, const uint32_t* __restrict__ resid_in,
   }
   // Each thread reads back only the words it wrote: no barrier needed.
   const int ng = 2 * e.num_digits;
-  for (int pi = 0; pi < c.r; ++pi) {
+  for (int pi = blockIdx.z; pi < c.r; pi += gridDim.z) {
     const uint32_t p = c.p[pi];
     const uint32_t pinv = c.pinv[pi];
     const uint2* tab16 = c.tables16 + static_cast<size_t>(pi) * 2 * d;

@@ -771,6 +771,25 @@ inline int64_t Ext16Min(const inspire_pir_server* s, int d) {
   return static_cast<int64_t>(s->sms) * std::max(1, 4096 / d);
 }
 
+// How ext_step16_kernel shares the r primes of `ciphertexts` (shard, request)
+// pairs at d = 8192, where a block has an SM to itself: the fewest blocks per
+// pair with the fewest transforms' turns (rounds of blocks times primes per
+// block). ext_step_kernel, a block per prime on the transforms of ntt.cuh, took
+// 137 us where this takes 105 for one ciphertext over Z_2^64, 374 where it takes
+// 284 for 64.
+inline int Ext16Split(const inspire_pir_server* s, int64_t ciphertexts, int r) {
+  int best = 1;
+  int64_t least = INT64_MAX;
+  for (int z = 1; z <= r; ++z) {
+    const int64_t turns = (ciphertexts * z + s->sms - 1) / s->sms * ((r + z - 1) / z);
+    if (turns < least) {
+      least = turns;
+      best = z;
+    }
+  }
+  return best;
+}
+
 // y_h = packing_key[k..2k): forward NTT over the finalize primes.
 template <typename T>
 NttRows<T> YhRows(const inspire_pir_server* s, Workspace* w, const T* pkey) {
@@ -843,7 +862,11 @@ Status FinalizeStage(inspire_pir_server* s, Workspace* w, int batch,
                        : PackedOut<T>{pairs + d, int64_t{2} * d, s->a_tilde.get<T>()};
   const int log_q = s->prm.log_modulus;
   if (!yh_done) RETURN_IF_ERROR(YhTransform<T>(s, w, batch, pkey, st));
-  if (s->ctx_f.tables16 != nullptr && static_cast<int64_t>(l) * t * batch >= s->sms) {
+  if (s->ctx_f.tables16 != nullptr &&
+      (d > 4096 || static_cast<int64_t>(l) * t * batch >= s->sms)) {
+    // d = 8192 at any number: its 512 threads fill an SM and beat the 1024 of
+    // finalize_kernel, whose transforms reduce in every butterfly (one request
+    // over Z_2^64, four primes: an answer 315 -> 287 us).
     const NttCtx& c = s->ctx_f;
     const size_t smem = static_cast<size_t>(c.r + 1) * d * 4;
     INSPIRE_NTT16_DISPATCH(
@@ -852,7 +875,7 @@ Status FinalizeStage(inspire_pir_server* s, Workspace* w, int batch,
             s->th_ntt.get<uint32_t>(), w->yh.get<uint32_t>(), k, gemv, nullptr, s->rows,
             packed, log_q, c));
     RETURN_IF_ERROR(Cuda(cudaGetLastError(), "finalize"));
-  } else if (s->ctx_f.tables16 != nullptr && d <= 4096) {
+  } else if (s->ctx_f.tables16 != nullptr) {
     // Several transform groups per block.
     const NttCtx& c = s->ctx_f;
     INSPIRE_NTT16_PAIR_DISPATCH(
@@ -958,20 +981,23 @@ Status RunPolyStage(inspire_pir_server* s, Workspace* w, int batch,
     ExtArgs e{log_q, s->prm.eval_log_digit, ne,
               LiveDigits(log_q, s->prm.eval_log_digit, ne), s->umask_e};
     const size_t smem = static_cast<size_t>(d) * 4 + 2ull * d * sizeof(T);
-    if (c.tables16 != nullptr && static_cast<int64_t>(l) * batch >= Ext16Min(s, d)) {
-      // Enough requests to fill the GPU with one block per (shard, request).
+    if (c.tables16 != nullptr &&
+        (d > 4096 || static_cast<int64_t>(l) * batch >= Ext16Min(s, d))) {
+      // Enough requests to fill the GPU with one block per (shard, request);
+      // d = 8192 at any number.
+      const unsigned z = d > 4096 ? Ext16Split(s, static_cast<int64_t>(l) * batch, c.r) : 1;
       INSPIRE_NTT16_DISPATCH(
           c.logd, RETURN_IF_ERROR(SetSmem(ext_step16_kernel<T, LG>, smem));
           for (int i = t - 2; i >= 0; --i) {
             const bool first = i == t - 2;
-            ext_step16_kernel<T, LG><<<dim3(l, batch), Ntt16<LG>::kThreads, smem, st>>>(
+            ext_step16_kernel<T, LG><<<dim3(l, batch, z), Ntt16<LG>::kThreads, smem, st>>>(
                 first, first ? nullptr : resid[(i + 1) & 1], resid[i & 1],
                 a_tilde + static_cast<int64_t>(i + 1) * d, 0, a_stride,
                 packed + static_cast<int64_t>(i + 1) * d, b_qstride, a_stride,
                 s->rgswa_ntt.get<uint32_t>(), 0, w->rgswb.get<uint32_t>(), e, c);
             RETURN_IF_ERROR(Cuda(cudaGetLastError(), "external product"));
           });
-    } else if (c.tables16 != nullptr && d <= 4096) {
+    } else if (c.tables16 != nullptr) {
       // Few requests: one block per prime, transforms side by side.
       const int64_t blocks = static_cast<int64_t>(c.r) * l * batch;
       INSPIRE_NTT16_PAIR_DISPATCH(
@@ -1346,14 +1372,15 @@ Status ExternalOnDevice(inspire_pir_server* s, Workspace* w, int batch,
     const size_t smem = static_cast<size_t>(d) * 4 + 2ull * d * sizeof(T);
     const T* cta = static_cast<const T*>(ct);
     const int64_t rq = static_cast<int64_t>(ng) * c.r * d;  // RGSW a per request
-    if (c.tables16 != nullptr && batch >= Ext16Min(s, d)) {
+    if (c.tables16 != nullptr && (d > 4096 || batch >= Ext16Min(s, d))) {
       // The radix-16 kernels as in RunPolyStage: one block per ciphertext.
+      const unsigned z = d > 4096 ? Ext16Split(s, batch, c.r) : 1;
       INSPIRE_NTT16_DISPATCH(
           c.logd, RETURN_IF_ERROR(SetSmem(ext_step16_kernel<T, LG>, smem));
-          ext_step16_kernel<T, LG><<<dim3(1, batch), Ntt16<LG>::kThreads, smem, st>>>(
+          ext_step16_kernel<T, LG><<<dim3(1, batch, z), Ntt16<LG>::kThreads, smem, st>>>(
               true, nullptr, w->resid0.get<uint32_t>(), cta, 2 * d, 0, cta + d, 2 * d, 0,
               w->rgswa.get<uint32_t>(), rq, w->rgswb.get<uint32_t>(), e, c));
-    } else if (c.tables16 != nullptr && d <= 4096) {
+    } else if (c.tables16 != nullptr) {
       INSPIRE_NTT16_PAIR_DISPATCH(
           c.logd, RETURN_IF_ERROR((LaunchPairExt<T, LG>(
                       static_cast<int64_t>(c.r) * batch, s->sms, dim3(c.r, 1, batch), st,

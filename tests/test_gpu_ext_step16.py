@@ -69,3 +69,37 @@ def test_radix16_external_product_matches_small_batches_and_oracle(
                                     mat.t_vec_h, mat.second_dim_a, fd[i], sd[i],
                                     pk[i])
         assert np.array_equal(big[i], want), i
+
+
+@pytest.mark.parametrize("coeff_bits,log_q,batch", [
+    (32, 32, 1), (32, 32, 60), (32, 32, 140), (64, 52, 1), (64, 52, 50),
+    (64, 52, 37), (64, 64, 120)])
+def test_primes_shared_by_blocks_at_d8192(coeff_bits, log_q, batch):
+    # Few ciphertexts: one to r blocks for the r primes of each.
+    import torch
+    d, ne = 8192, 3
+    params = synthetic.make_params(d=d, n=64, t=1, coeff_bits=coeff_bits,
+                                   log_q=log_q)
+    mat = synthetic.make_material(params, seed=batch, db_cols=64)
+    srv = pir.PirServer.CreateCombined(params, mat.db, mat.pack, mat.a_tilde_agg,
+                                       mat.t_vec_h, None)
+    rng = np.random.default_rng(batch + log_q)
+    cdt = params.coeff_dtype
+    top = np.iinfo(cdt).max
+    ct = rng.integers(0, top, (batch, 2, d), dtype=cdt, endpoint=True)
+    rgsw = rng.integers(0, top, (batch, 2 * ne, 2, d), dtype=cdt, endpoint=True)
+    ct[-1, 0] = top
+    rgsw[-1] = top
+    view = np.int32 if coeff_bits == 32 else np.int64
+    t_ct, t_rg = (torch.from_numpy(x.view(view)).cuda() for x in (ct, rgsw))
+    out = torch.empty_like(t_ct)
+    srv.external_product_device(batch, t_ct.data_ptr(), t_rg.data_ptr(),
+                                out.data_ptr())
+    torch.cuda.synchronize()
+    got = out.cpu().numpy().view(cdt)
+    op = _oparams(params)
+    for i in sorted({0, batch // 2, batch - 1}):
+        wa, wb = orc.external_product(op, ct[i, 0], ct[i, 1],
+                                      rgsw[i].reshape(-1, d))
+        assert np.array_equal(got[i, 0], wa), i
+        assert np.array_equal(got[i, 1], wb), i
