@@ -152,7 +152,7 @@ constexpr int kFastR = 32;   // classes per block (one warp's lanes)
 // groups (64-byte row pieces; a 64 KB tile of 16-bit values at t = 8, two
 // blocks per SM, as the registers of the t = 8 transform allow); wider
 // values 16, which keeps the tile within a block's limit.
-template <typename V>
+template <typename V, int T>
 struct FastShape {
   static constexpr int kG = sizeof(V) <= 2 ? 32 : 16;
   static constexpr int kGW = 8;
@@ -160,13 +160,18 @@ struct FastShape {
   // words) are permuted instead: word w of class c sits at w ^ (c / 2), so 32
   // classes' writes of one word and the store phase's reads of consecutive
   // words both touch 32 banks. (Padded to 80 bytes for 16-byte reads, the
-  // writes took four passes each.)
-  static constexpr int kRow = sizeof(V) == 2 ? kG : kG + 1;
-  __device__ static __forceinline__ int swizzle(int c) { return (c >> 1) & 15; }
+  // writes took four passes each.) At t = 2 a thread writes two words a
+  // pair of groups and the reads weigh more: padded rows, 92.7 -> 89.8 us at
+  // 40000 records of 2048.
+  static constexpr bool kPermuted = sizeof(V) == 2 && T > 2;
+  static constexpr int kRow = kPermuted ? kG : kG + (sizeof(V) == 2 ? 8 : 1);
+  __device__ static __forceinline__ int swizzle(int c) {
+    return kPermuted ? (c >> 1) & 15 : 0;
+  }
   // Index of (tile row rm, class c, group g).
   __device__ static __forceinline__ int at(int rm, int c, int g) {
     const int row = rm * kFastR + c;
-    if constexpr (sizeof(V) == 2) {
+    if constexpr (kPermuted) {
       return row * kRow + 2 * ((g >> 1) ^ swizzle(c)) + (g & 1);
     } else {
       return row * kRow + g;
@@ -313,7 +318,7 @@ __device__ __forceinline__ void lazy_tile_store(const uint32_t (&xa)[T][T / 2],
   for (int r = 0; r < T; ++r) {
 #pragma unroll
     for (int m = 0; m < H; ++m) {
-      V* dst = tile + FastShape<V>::at(r * H + m, c0, gi);
+      V* dst = tile + FastShape<V, T>::at(r * H + m, c0, gi);
       if constexpr (sizeof(V) == 2) {
         if (hb) {
           *reinterpret_cast<uint32_t*>(dst) = xa[r][m] | (xb[r][m] << 16);
@@ -336,13 +341,13 @@ __device__ __forceinline__ void lazy_tile_store(const uint32_t (&xa)[T][T / 2],
 // that bound (Shoup, valid for any 32-bit operand), gives the same residue
 // as reducing after every step. Used when 2 * lazy_off < 2^32 and p < 2^31.
 template <typename V, int T, bool SMALL, bool LAZY = false>
-__global__ void __launch_bounds__(kFastR * FastShape<V>::kGW)
+__global__ void __launch_bounds__(kFastR * FastShape<V, T>::kGW)
 interpolate_fast_kernel(const V* __restrict__ raw, InterpArgs a, ModConsts mc,
                         V* __restrict__ out) {
   constexpr int H = T / 2;
   constexpr int LOGT = T == 2 ? 1 : (T == 4 ? 2 : 3);
-  constexpr int kFastG = FastShape<V>::kG;
-  constexpr int kFastGW = FastShape<V>::kGW;
+  constexpr int kFastG = FastShape<V, T>::kG;
+  constexpr int kFastGW = FastShape<V, T>::kGW;
   // [T*H rows][kFastR classes][groups] (dynamic shared memory)
   extern __shared__ __align__(16) unsigned char tile_raw[];
   V* tile = reinterpret_cast<V*>(tile_raw);
@@ -425,7 +430,7 @@ interpolate_fast_kernel(const V* __restrict__ raw, InterpArgs a, ModConsts mc,
     for (int r = 0; r < T; ++r) {
 #pragma unroll
       for (int m = 0; m < H; ++m) {
-        tile[FastShape<V>::at(r * H + m, c0, gi)] =
+        tile[FastShape<V, T>::at(r * H + m, c0, gi)] =
             static_cast<V>(scale_p<SMALL>(x[r][m], a.tinv, p, mc));
       }
     }
@@ -435,6 +440,7 @@ interpolate_fast_kernel(const V* __restrict__ raw, InterpArgs a, ModConsts mc,
   // Stores: kFastG consecutive columns of each DB row.
   const int64_t left = a.groups - g_base;
   const int G = left < kFastG ? static_cast<int>(left) : kFastG;
+  constexpr int kThreads = kFastR * kFastGW;
   if constexpr (sizeof(V) == 2) {
     if ((a.out_cols & 7) == 0 && G == kFastG &&
         (reinterpret_cast<uintptr_t>(out) & 15) == 0) {
@@ -443,7 +449,6 @@ interpolate_fast_kernel(const V* __restrict__ raw, InterpArgs a, ModConsts mc,
       // multiple of 32). Thread i writes
       // chunk i % 4 of class (i / 4) % 32, tile rows i / 128 + 2 j.
       constexpr int kChunks = kFastG / 8;
-      constexpr int kThreads = kFastR * kFastGW;
       constexpr int kRmStep = kThreads / (kChunks * kFastR);
       constexpr int kIters = T * H / kRmStep;
       static_assert(kThreads % (kChunks * kFastR) == 0 && (T * H) % kRmStep == 0,
@@ -455,48 +460,58 @@ interpolate_fast_kernel(const V* __restrict__ raw, InterpArgs a, ModConsts mc,
       const int64_t ss = static_cast<int64_t>(a.s) * a.out_cols;
       V* dst = out + (static_cast<int64_t>(k) * T * a.d + c_start + c) * a.out_cols + g_base +
                8 * q;
-      const uint32_t* src = reinterpret_cast<const uint32_t*>(tile) + c * (kFastG / 2);
-      const int swz = FastShape<V>::swizzle(c);
+      constexpr int kWords = FastShape<V, T>::kRow / 2;  // a row's words
+      const uint32_t* src = reinterpret_cast<const uint32_t*>(tile) + c * kWords;
+      const int swz = FastShape<V, T>::swizzle(c);
 #pragma unroll
       for (int j = 0; j < kIters; ++j) {
         const int rm = rm0 + kRmStep * j;
         const int r = rm / H, m = rm % H;
-        const uint32_t* w = src + rm * kFastR * (kFastG / 2);
-        const uint4 v = make_uint4(w[(4 * q) ^ swz], w[(4 * q + 1) ^ swz],
-                                   w[(4 * q + 2) ^ swz], w[(4 * q + 3) ^ swz]);
+        const uint32_t* w = src + rm * kFastR * kWords;
+        const uint4 v = FastShape<V, T>::kPermuted
+                            ? make_uint4(w[(4 * q) ^ swz], w[(4 * q + 1) ^ swz],
+                                         w[(4 * q + 2) ^ swz], w[(4 * q + 3) ^ swz])
+                            : *reinterpret_cast<const uint4*>(w + 4 * q);
         *reinterpret_cast<uint4*>(dst + r * ds + m * ss) = v;
       }
       return;
     }
+  }
+  const int64_t ds = static_cast<int64_t>(a.d) * a.out_cols;
+  const int64_t ss = static_cast<int64_t>(a.s) * a.out_cols;
+  V* base = out + (static_cast<int64_t>(k) * T * a.d + c_start) * a.out_cols + g_base;
+  if constexpr (sizeof(V) == 2) {
     if ((a.out_cols & 1) == 0 && G == kFastG &&
         (reinterpret_cast<uintptr_t>(out) & 3) == 0) {
       // Two neighbouring groups per 32-bit store (g_base a multiple of 32:
       // every store is 4-byte aligned).
       constexpr int kPairs = kFastG / 2;
-      for (int idx = threadIdx.x; idx < T * H * kFastR * kPairs; idx += blockDim.x) {
-        const int gp = idx % kPairs;
-        const int c = (idx / kPairs) % kFastR;
-        const int rm = idx / (kPairs * kFastR);
-        const int r = rm / H, m = rm % H;
-        const int64_t row = static_cast<int64_t>(k) * T * a.d +
-                            static_cast<int64_t>(r) * a.d + c_start + c +
-                            static_cast<int64_t>(m) * a.s;
-        const uint32_t v =
-            *reinterpret_cast<const uint32_t*>(tile + FastShape<V>::at(rm, c, 2 * gp));
-        *reinterpret_cast<uint32_t*>(out + row * a.out_cols + g_base + 2 * gp) = v;
+      constexpr int kStep = kThreads / kPairs;  // classes at a time
+      const int gp = threadIdx.x % kPairs;
+#pragma unroll
+      for (int i = 0; i < kFastR / kStep; ++i) {
+        const int c = threadIdx.x / kPairs + i * kStep;
+        V* dst = base + static_cast<int64_t>(c) * a.out_cols + 2 * gp;
+#pragma unroll
+        for (int rm = 0; rm < T * H; ++rm) {
+          *reinterpret_cast<uint32_t*>(dst + rm / H * ds + rm % H * ss) =
+              *reinterpret_cast<const uint32_t*>(tile + FastShape<V, T>::at(rm, c, 2 * gp));
+        }
       }
       return;
     }
   }
-  for (int idx = threadIdx.x; idx < T * H * kFastR * kFastG; idx += blockDim.x) {
-    const int g = idx % kFastG;
-    const int c = (idx / kFastG) % kFastR;
-    const int rm = idx / (kFastG * kFastR);
-    if (g >= G) continue;
-    const int r = rm / H, m = rm % H;
-    const int64_t row = static_cast<int64_t>(k) * T * a.d + static_cast<int64_t>(r) * a.d +
-                        c_start + c + static_cast<int64_t>(m) * a.s;
-    out[row * a.out_cols + g_base + g] = tile[FastShape<V>::at(rm, c, g)];
+  constexpr int kStep = kThreads / kFastG;
+  const int g = threadIdx.x % kFastG;
+  if (g >= G) return;
+#pragma unroll
+  for (int i = 0; i < kFastR / kStep; ++i) {
+    const int c = threadIdx.x / kFastG + i * kStep;
+    V* dst = base + static_cast<int64_t>(c) * a.out_cols + g;
+#pragma unroll
+    for (int rm = 0; rm < T * H; ++rm) {
+      dst[rm / H * ds + rm % H * ss] = tile[FastShape<V, T>::at(rm, c, g)];
+    }
   }
 }
 
@@ -603,12 +618,12 @@ int Run(const V* raw, int64_t n, int d, int t, int l, uint32_t p, V* out,
       const uint64_t off = (bound + p - 1) / p * p;
       const bool lazy = sizeof(V) <= 2 && small && 2 * off < (1ull << 31);
       a.lazy_off = static_cast<uint32_t>(lazy ? off : 0);
-      constexpr int kFastG = FastShape<V>::kG;
+      constexpr int kFastG = FastShape<V, 8>::kG;
       dim3 grid(static_cast<unsigned>(a.s / kFastR),
                 static_cast<unsigned>((groups + kFastG - 1) / kFastG), static_cast<unsigned>(l));
-      const int threads = kFastR * FastShape<V>::kGW;
-      const size_t smem =
-          static_cast<size_t>(t) * (t / 2) * kFastR * FastShape<V>::kRow * sizeof(V);
+      const int threads = kFastR * FastShape<V, 8>::kGW;
+      const int row = t == 2 ? FastShape<V, 2>::kRow : FastShape<V, 8>::kRow;
+      const size_t smem = static_cast<size_t>(t) * (t / 2) * kFastR * row * sizeof(V);
       auto launch = [&](auto kernel) {
         cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              static_cast<int>(smem));
