@@ -57,3 +57,10 @@ def test_one_slice_server_with_wide_digits(evalg):
     # Products of 116 and 109 bits: five 27-bit primes, where the answers of
     # the same server take four.
     test_matches_oracle(2048, 64, 64, evalg, 2)
+
+
+@pytest.mark.parametrize("d,evalg", [(2048, (4, 6)), (2048, (4, 7)),
+                                     (4096, (2, 6)), (4096, (2, 16))])
+def test_narrow_digits_on_either_side_of_the_one_launch_form(d, evalg):
+    # Products of at most 51 bits: two primes where the one launch takes three.
+    test_matches_oracle(d, 32, 32, evalg, 3)
