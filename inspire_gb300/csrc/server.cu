@@ -1043,6 +1043,13 @@ Status RunPolyStage(inspire_pir_server* s, Workspace* w, int batch,
   return Status{};
 }
 
+// Residues of one Horner step, of which the launches per step keep two: a
+// server whose answers and external products both run in one launch has none.
+int64_t ResidBytes(const inspire_pir_server* s, int batch) {
+  const bool steps = !s->fused_poly || (s->eval_rule.ok() && !s->fused_ext);
+  return steps ? static_cast<int64_t>(batch) * s->l * s->ctx_e.r * 2 * s->d * 4 : 0;
+}
+
 int64_t WorkspaceBytes(const inspire_pir_server* s, int batch) {
   const int64_t w = Words(s->prm.coeff_bits);
   const int64_t d = s->d;
@@ -1051,7 +1058,7 @@ int64_t WorkspaceBytes(const inspire_pir_server* s, int batch) {
               B * std::max(1, 2 * s->ne) * d * w + B * s->rows * w +
               B * s->k * s->ctx_f.r * d * 4 +
               B * std::max(1, 2 * s->ne) * s->ctx_e.r * d * 4 +
-              B * s->l * s->t * d * w + 2 * B * s->l * s->ctx_e.r * 2 * d * 4 +
+              B * s->l * s->t * d * w + 2 * ResidBytes(s, batch) +
               B * s->l * 2 * d * w;
   if (s->limb) b += s->limb->ScratchBytes(batch);
   return b;
@@ -1069,8 +1076,8 @@ Status EnsureWorkspace(inspire_pir_server* s, Workspace* ws, int batch) {
   RETURN_IF_ERROR(ws->yh.Alloc(B * s->k * s->ctx_f.r * d * 4));
   RETURN_IF_ERROR(ws->rgswb.Alloc(B * std::max(1, 2 * s->ne) * s->ctx_e.r * d * 4));
   RETURN_IF_ERROR(ws->packed.Alloc(B * s->l * s->t * d * w));
-  RETURN_IF_ERROR(ws->resid0.Alloc(B * s->l * s->ctx_e.r * 2 * d * 4));
-  RETURN_IF_ERROR(ws->resid1.Alloc(B * s->l * s->ctx_e.r * 2 * d * 4));
+  RETURN_IF_ERROR(ws->resid0.Alloc(ResidBytes(s, batch)));
+  RETURN_IF_ERROR(ws->resid1.Alloc(ResidBytes(s, batch)));
   RETURN_IF_ERROR(ws->resp.Alloc(B * s->l * 2 * d * w));
   if (s->limb && !ws->limb) ws->limb = s->limb->NewScratch();
   ws->cap = batch;
