@@ -2,9 +2,10 @@
 //
 // The reference multiplies polynomials with an FP64 FFT over 2d points and
 // rounds (crypto/polynomial_fft.cc:68-197). On the GPU the same integer
-// result is produced exactly with a negacyclic NTT over a few 31-bit primes
-// p = c * 2^16 + 1 (so a primitive 2d-th root of unity exists for d <= 2^15)
-// followed by a Garner CRT reconstruction mod 2^w. All arithmetic is 32-bit:
+// result is produced exactly with a negacyclic NTT over a few primes of 31 bits,
+// p = c * 2^16 + 1, or of 27 bits, p = c * 2^14 + 1 (a primitive 2d-th root of
+// unity exists for d <= 2^15 or 2^13), followed by a CRT reconstruction
+// mod 2^w. All arithmetic is 32-bit:
 //   * Shoup multiplication by precomputed constants (twiddles, scalings),
 //   * signed Montgomery multiplication for variable x variable products.
 #pragma once

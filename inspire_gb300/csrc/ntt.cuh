@@ -1,4 +1,5 @@
-// Block-level negacyclic NTT over one 31-bit prime and the Garner CRT that
+// Block-level negacyclic NTT over one prime (of 31 bits, or of 27 where the ring
+// also has the radix-16 transforms) and the Garner CRT that
 // turns r residues back into an integer mod 2^w.
 //
 // Forward: Cooley-Tukey with the psi-twisted twiddles merged in (natural
@@ -303,32 +304,6 @@ __device__ __forceinline__ void ntt_inverse_t(uint32_t* a, const NttCtx& c,
 // Garner reconstruction: x[i] < p_i -> the integer in
 // [-(p_{r-1}-1)/2 * P', (p_{r-1}+1)/2 * P') (P' = product of the other
 // primes) congruent to x, reduced mod 2^w.
-// The same for R primes known at compile time (a third of the code).
-template <typename T, int R>
-__device__ __forceinline__ T crt_fixed(const uint32_t (&x)[R], const NttCtx& c) {
-  uint32_t a[R];
-  a[0] = x[0];
-#pragma unroll
-  for (int i = 1; i < R; ++i) {
-    const uint32_t p = c.p[i];
-    uint32_t v = x[i];
-#pragma unroll
-    for (int j = 0; j < i; ++j) {
-      const uint32_t aj = umin32(a[j], a[j] - p);
-      v = mont_mul(umin32(v - aj, v - aj + p), c.garner[j][i], p, c.pinv[i]);
-    }
-    a[i] = v;
-  }
-  // A top digit above the half counts as negative.
-  T acc = static_cast<T>(a[R - 1]) * static_cast<T>(c.pm[R - 1]);
-  if (a[R - 1] > c.half[R - 1]) {
-    acc -= static_cast<T>(c.p[R - 1]) * static_cast<T>(c.pm[R - 1]);
-  }
-#pragma unroll
-  for (int i = 0; i + 1 < R; ++i) acc += static_cast<T>(a[i]) * static_cast<T>(c.pm[i]);
-  return acc;
-}
-
 template <typename T>
 __device__ __forceinline__ T crt_reconstruct(const uint32_t (&x)[kMaxPrimes],
                                              const NttCtx& c) {

@@ -63,11 +63,6 @@ struct Ntt16 {
     for (int i = 0; i < w; ++i) b += 15 << (4 * i);
     return b;
   }
-  // Slot of W[m0 2^s + g 2^s + x] (window w, stage s) in the permuted table.
-  __host__ __device__ static constexpr int Slot(int w, int s, int x, int g) {
-    return Base(w) + (1 << Start(w)) * ((1 << s) - (1 << Skip(w))) +
-           x * (1 << Start(w)) + g;
-  }
 };
 
 #ifdef __CUDACC__

@@ -263,7 +263,7 @@ struct RootPowers {
 
 // Every prime's tables [W | W shoup | IW | IW shoup], W[i] = psi^brv(i), and
 // for d = 2^11..2^13 the same words in the window order of the radix-16
-// transforms (Ntt16<LOGD>::Slot) after all the plain ones. One thread per
+// transforms (`slot` below) after all the plain ones. One thread per
 // twiddle pair: at most log d - 1 dependent Shoup products and two 32-bit
 // quotients, so the launch takes a few microseconds; built by the host
 // (PowMod per entry, permutation, copy) the tables took 3.2 ms at d = 4096,
