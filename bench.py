@@ -857,7 +857,7 @@ def run_single_workload(args):
                      "kernel": "fused_gemv", "ms": ms_prod, "bytes": alg,
                      "peak_kind": peak_kind + " copy"},
         "clocks": clk.summary(),
-        "gpu_launches": profiling.launches_per_step(pir.ENGINE_PLAIN, t) * args.steps,
+        "gpu_launches": profiling.launches_per_step(pir.ENGINE_PLAIN, t, d) * args.steps,
         "e2e": {"value": 1000.0 / statistics.mean(t_e2e), "unit": "queries/s",
                 "latency_ms_p50": pct(t_e2e, 0.5),
                 "h2d_bytes_per_step": int(h_fd[0].nbytes + h_sd[0].nbytes +

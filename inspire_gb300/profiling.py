@@ -66,12 +66,15 @@ LIMB64_TRAFFIC_PER_UNIT = (3.490142e9 + 0.163364e9) / (16384 * 40960)
 GEMV_TRAFFIC_PER_ALG_BYTE = (3.221e9 + 2.9e6) / 3.222e9
 
 
-def launches_per_step(engine, t):
-    # Answers at d = 2048 and 4096: the products (the fused GEMV, or the
-    # tensor engine's query-digit split, pack-key digit split and limb GEMM),
-    # NTT(y_h), NTT(rgsw) and the polynomial stage in one launch.
+def launches_per_step(engine, t, d):
+    # An answer with the workloads' 19-bit gadgets: the products (the fused
+    # GEMV, or the tensor engine's query-digit split, pack-key digit split and
+    # limb GEMM), the request transforms (y_h and, for t > 1, the RGSW rows) in
+    # one launch, and the polynomial stage: one launch at d = 2048 and 4096, at
+    # other degrees finalize, t - 1 external products and the modulus switch.
     products = 3 if engine == pir.ENGINE_TENSOR else 1
-    return products + 1 + (1 if t > 1 else 0) + 1
+    poly = 1 if d in (2048, 4096) else 1 + (t - 1) + 1
+    return products + 1 + poly
 
 
 def kernel_times(srv, engine, batch, t_fd, t_sd, t_pk, t_out, stream, n1,
@@ -136,5 +139,5 @@ def kernel_times(srv, engine, batch, t_fd, t_sd, t_pk, t_out, stream, n1,
                 "traffic_source": "ncu small case scaled by algorithmic bytes",
                 "kernel": "fused_gemv", "peak_kind": kind + " copy"}
     return {"roofline": roof, "kernels": kernels,
-            "launches_per_step": launches_per_step(engine,
-                                                   srv.params.interpolation_degree)}
+            "launches_per_step": launches_per_step(
+                engine, srv.params.interpolation_degree, srv.params.rlwe.degree)}

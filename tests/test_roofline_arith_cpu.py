@@ -41,3 +41,15 @@ def test_headline_counts():
     assert profiling.plain_bytes(R, C, K) == 9_664_364_544
     # C1: n = 4096, d = 2048, t = 2 over Z_2^64 (u64 words).
     assert profiling.plain_bytes(4096, 2048, 4096, word=8) == 83_968_000
+
+
+@pytest.mark.parametrize("engine,t,d,launches", [
+    ("tensor", 8, 4096, 5),   # two digit splits, GEMM, transforms, one stage
+    ("plain", 2, 2048, 3), ("plain", 1, 2048, 3), ("plain", 4, 2048, 3),
+    # finalize, t - 1 external products and the modulus switch apart
+    ("plain", 2, 8192, 5), ("tensor", 2, 8192, 7), ("plain", 4, 1024, 7),
+    ("plain", 1, 512, 4)])
+def test_launches_of_an_answer(engine, t, d, launches):
+    from inspire_gb300 import pir
+    kind = pir.ENGINE_TENSOR if engine == "tensor" else pir.ENGINE_PLAIN
+    assert profiling.launches_per_step(kind, t, d) == launches
