@@ -474,7 +474,12 @@ int inspire_pir_server_shape(const inspire_pir_server* server, int64_t* rows,
                              int64_t* db_cols, int64_t* pack_cols);
 
 /* GetDbMultiplyTime / GetPackingTime / GetPolyEvalTime
- * (crypto/pir/server/pir_server.h:70-72), accumulated in milliseconds. */
+ * (crypto/pir/server/pir_server.h:70-72), accumulated in milliseconds over the
+ * calls with host buffers. The launches do not split as the reference's stages
+ * do: db_mult_ms is both matrix products (database and pack matrix), and where
+ * the polynomial stage is one launch (d = 2048 and 4096) FinalizeMatrixPack runs
+ * inside it, so that poly_eval_ms holds its time and packing_ms is near zero.
+ * The three add up to the answer's time on the device. */
 int inspire_pir_server_timings(const inspire_pir_server* server,
                                double* db_mult_ms, double* packing_ms,
                                double* poly_eval_ms);

@@ -187,6 +187,7 @@ class PirServer {
 
   // Accumulated times in milliseconds (the reference returns absl::Duration).
   double GetDbMultiplyTime() const { return Times()[0]; }
+  // Near zero where the polynomial stage is one launch (inspire_pir.h).
   double GetPackingTime() const { return Times()[1]; }
   double GetPolyEvalTime() const { return Times()[2]; }
 

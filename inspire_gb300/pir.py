@@ -542,13 +542,17 @@ class PirServer:
         return a.value, b.value, c.value
 
     def GetDbMultiplyTime(self):
-        """Accumulated DB product time in milliseconds."""
+        """Accumulated time of both matrix products in milliseconds."""
         return self._timings()[0]
 
     def GetPackingTime(self):
+        """FinalizeMatrixPack; near zero at d = 2048 and 4096, where it runs
+        inside the polynomial stage's one launch."""
         return self._timings()[1]
 
     def GetPolyEvalTime(self):
+        """EvalPoly and the modulus switch (and FinalizeMatrixPack where the
+        polynomial stage is one launch)."""
         return self._timings()[2]
 
 
