@@ -50,3 +50,17 @@ def test_matches_oracle(case):
                                     m.t_vec_h, m.second_dim_a, fd[i], sd[i],
                                     pk[i])
         assert np.array_equal(got[i], want), i
+
+
+@pytest.mark.parametrize("case", [
+    # One digit of 30 bits, above the 27-bit primes, in the one launch.
+    (2048, 2, 1, 32, 32, (19, 2), (30, 1), 2),
+    (4096, 4, 1, 32, 32, (19, 2), (29, 1), 2),
+    # Eight live digits on six groups: a second round of two.
+    (2048, 4, 1, 64, 64, (19, 2), (16, 4), 2),
+    (2048, 2, 2, 64, 52, (19, 2), (13, 4), 1),
+    # d = 4096 over Z_2^64: eight live digits on three groups.
+    (4096, 2, 1, 64, 64, (19, 2), (16, 4), 1),
+], ids=str)
+def test_wide_digits_and_second_rounds(case):
+    test_matches_oracle(case)
