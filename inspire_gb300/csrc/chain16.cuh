@@ -37,14 +37,14 @@ constexpr size_t Chain16Smem(int k, int side) {
 }
 
 #ifdef __CUDACC__
-// grid = (2 R, slices), clusters of R, G d / 16 threads, side digits side by
-// side (Chain16Smem). Needs log_digit <= 27
+// grid = (2 R, slices), clusters of R, G d / 16 threads, SIDE digits side by
+// side (compiled in: as an argument it cost the links of d = 2048 2 %). Needs log_digit <= 27
 // and at most 30 digits. Outputs as pp_chain_kernel's.
-template <typename T, int LOGD, int G, int R>
+template <typename T, int LOGD, int G, int R, int SIDE>
 __global__ void __launch_bounds__(G * Ntt16<LOGD>::kThreads, 1)
 chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainArgs a,
                        const __grid_constant__ NttCtx c, const __grid_constant__ CrtArgs crt,
-                       int side, T* __restrict__ tg, T* __restrict__ tgh, T* __restrict__ fin) {
+                       T* __restrict__ tg, T* __restrict__ tgh, T* __restrict__ fin) {
   extern __shared__ __align__(16) uint32_t smem[];
   constexpr int d = Ntt16<LOGD>::kD;
   constexpr int NT = Ntt16<LOGD>::kThreads;
@@ -52,7 +52,7 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
   constexpr int kQuads = (d / 4 + kThreads - 1) / kThreads;
   constexpr int kWords = (d + kThreads - 1) / kThreads;
   constexpr bool kLocal = LOGD <= 12;  // twiddles and key parts in shared memory
-  static_assert(G >= kChainSide, "a group per digit");
+  static_assert(SIDE <= kChainSide && G >= SIDE, "a group per digit");
   using S = typename std::make_signed<T>::type;
   const int tid = threadIdx.x;
   const int grp = tid / NT;
@@ -68,9 +68,9 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
   const uint2* itw = tw + d;
   const int w_stride = kLocal ? d : R * d;
   const uint32_t* W = kLocal ? smem + 4 * d : a.Wg + pi * d;        // [k][w_stride]
-  uint32_t* regions = smem + (kLocal ? (4 + k) * d : 0);            // [side][d]
+  uint32_t* regions = smem + (kLocal ? (4 + k) * d : 0);            // [SIDE][d]
   uint32_t* region = regions + grp * d;
-  uint32_t* res = regions + side * d;
+  uint32_t* res = regions + SIDE * d;
   int32_t* dig = reinterpret_cast<int32_t*>(res + d);      // [k][d]
   if constexpr (kLocal) {
     const uint4* src = reinterpret_cast<const uint4*>(tables);
@@ -137,8 +137,8 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
     }
     uint32_t x[16];
 #pragma unroll 1
-    for (int l0 = 0; l0 < k; l0 += side) {
-      if (grp < side && l0 + grp < k) {
+    for (int l0 = 0; l0 < k; l0 += SIDE) {
+      if (grp < SIDE && l0 + grp < k) {
         const int32_t* src = dig + (l0 + grp) * d + lt;
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
@@ -161,8 +161,8 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
             const int from = pp_bitrev(((power * odd) & (2 * d - 1)) >> 1, LOGD);
             const int at = ntt16_pos<LOGD>(e + m);
 #pragma unroll
-            for (int o = 0; o < kChainSide; ++o) {
-              if (o < side && l0 + o < k) {
+            for (int o = 0; o < SIDE; ++o) {
+              if (l0 + o < k) {
                 const uint32_t* w = W + (l0 + o) * w_stride + from;
                 sum[u][m] += static_cast<uint64_t>(regions[o * d + at]) *
                              (kLocal ? *w : __ldg(w));
@@ -171,7 +171,7 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
           }
         }
       }
-      if (l0 + side < k) __syncthreads();
+      if (l0 + SIDE < k) __syncthreads();
     }
 #pragma unroll
     for (int u = 0; u < kQuads; ++u) {

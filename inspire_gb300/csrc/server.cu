@@ -3994,11 +3994,11 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
           dfin.get<T>(), ca, c, static_cast<T*>(th_out), static_cast<T*>(a_out));
       return Cuda(cudaGetLastError(), "a_tilde_agg");
     };
-    auto chain_clusters = [&](auto ltag) -> Status {
+    auto chain_clusters = [&](auto ltag, auto stag) -> Status {
       constexpr int LG = decltype(ltag)::value;
       constexpr int GR = LG <= 12 ? 4 : 2;
       constexpr int R = AnswerPolyPrimes<T>();
-      auto* kernel = chain16_cluster_kernel<T, LG, GR, R>;
+      auto* kernel = chain16_cluster_kernel<T, LG, GR, R, decltype(stag)::value>;
       RETURN_IF_ERROR(SetSmem(kernel, cluster_smem));
       cudaLaunchAttribute cluster;
       cluster.id = cudaLaunchAttributeClusterDimension;
@@ -4013,7 +4013,7 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
       cfg.attrs = &cluster;
       cfg.numAttrs = 1;
       const CrtArgs crt = tabs->Crt(R);
-      RETURN_IF_ERROR(Cuda(cudaLaunchKernelEx(&cfg, kernel, ev->get<T>(), ca, c, crt, chain_side,
+      RETURN_IF_ERROR(Cuda(cudaLaunchKernelEx(&cfg, kernel, ev->get<T>(), ca, c, crt,
                                               dtg.get<T>(), dtgh.get<T>(), dfin.get<T>()),
                            "reduction chains"));
       constexpr int GT = LG == 11 ? 3 : LG == 12 ? 2 : 1;
@@ -4029,12 +4029,16 @@ int inspire_preprocess_matrix_pack(int32_t coeff_bits, int32_t mat_kind,
     using I5 = std::integral_constant<int, 5>;
     const int groups16 = logd == 11 ? std::min(r, 5) : logd == 12 ? std::min(r, 3) : 1;
     if (clusters && fits16) {
+      auto sides = [&](auto ltag) {
+        return chain_side == 1 ? chain_clusters(ltag, I1{}) : chain_clusters(ltag, I2{});
+      };
       if (logd == 11) {
-        RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 11>{}));
+        RETURN_IF_ERROR(sides(std::integral_constant<int, 11>{}));
       } else if (logd == 12) {
-        RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 12>{}));
+        RETURN_IF_ERROR(sides(std::integral_constant<int, 12>{}));
       } else if constexpr (sizeof(T) == 4) {
-        RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 13>{}));
+        // Gadgets that fits16 admits have room for two.
+        RETURN_IF_ERROR(chain_clusters(std::integral_constant<int, 13>{}, I2{}));
       }
     } else if (fits16 && logd == 11) {
       if (groups16 == 2) RETURN_IF_ERROR(chains16(std::integral_constant<int, 11>{}, I2{}));
