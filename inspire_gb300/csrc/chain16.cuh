@@ -38,8 +38,8 @@ constexpr size_t Chain16Smem(int k, int side) {
 
 #ifdef __CUDACC__
 // grid = (2 R, slices), clusters of R, G d / 16 threads, SIDE digits side by
-// side (compiled in: as an argument it cost the links of d = 2048 2 %). Needs log_digit <= 27
-// and at most 30 digits. Outputs as pp_chain_kernel's.
+// side (compiled in: as an argument it cost the links of d = 2048 2 %). Needs
+// log_digit <= 27 and at most 30 digits. Outputs as pp_chain_kernel's.
 template <typename T, int LOGD, int G, int R, int SIDE>
 __global__ void __launch_bounds__(G * Ntt16<LOGD>::kThreads, 1)
 chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainArgs a,
@@ -66,9 +66,8 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
   const uint2* tables = c.tables16 + static_cast<size_t>(pi) * 2 * d;
   const uint2* tw = kLocal ? reinterpret_cast<const uint2*>(smem) : tables;
   const uint2* itw = tw + d;
-  const int w_stride = kLocal ? d : R * d;
-  const uint32_t* W = kLocal ? smem + 4 * d : a.Wg + pi * d;        // [k][w_stride]
-  uint32_t* regions = smem + (kLocal ? (4 + k) * d : 0);            // [SIDE][d]
+  uint32_t* W = smem + 4 * d;                                       // [k][d] if kLocal
+  uint32_t* regions = kLocal ? W + static_cast<int64_t>(k) * d : smem;  // [SIDE][d]
   uint32_t* region = regions + grp * d;
   uint32_t* res = regions + SIDE * d;
   int32_t* dig = reinterpret_cast<int32_t*>(res + d);      // [k][d]
@@ -76,7 +75,7 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
     const uint4* src = reinterpret_cast<const uint4*>(tables);
     uint4* dst = reinterpret_cast<uint4*>(smem);
     for (int i = tid; i < d; i += kThreads) dst[i] = __ldg(src + i);
-    uint4* wd = reinterpret_cast<uint4*>(smem + 4 * d);
+    uint4* wd = reinterpret_cast<uint4*>(W);
     for (int i = tid; i < k * (d / 4); i += kThreads) {
       const int l = i / (d / 4);
       wd[i] = __ldg(reinterpret_cast<const uint4*>(
@@ -163,9 +162,13 @@ chain16_cluster_kernel(const T* __restrict__ ev, const __grid_constant__ ChainAr
 #pragma unroll
             for (int o = 0; o < SIDE; ++o) {
               if (l0 + o < k) {
-                const uint32_t* w = W + (l0 + o) * w_stride + from;
-                sum[u][m] += static_cast<uint64_t>(regions[o * d + at]) *
-                             (kLocal ? *w : __ldg(w));
+                uint32_t w;
+                if constexpr (kLocal) {
+                  w = W[(l0 + o) * d + from];
+                } else {
+                  w = __ldg(a.Wg + ((l0 + o) * R + pi) * d + from);
+                }
+                sum[u][m] += static_cast<uint64_t>(regions[o * d + at]) * w;
               }
             }
           }
