@@ -10,8 +10,9 @@
 // and row. The multiplier bounds the kernel (a butterfly takes four of the 64
 // slots a cycle, a 64-bit multiply-add three): n = 8 blocks of 4096 over Z_2^32
 // come to 37 thousand cycles per row, 3.9 ms for 32768 rows; the kernel takes
-// 7.1 ms (issue 57 % of cycles, spills at 128 registers), three primes with whole
-// words and a separate reconstruction took 13.
+// 7.1 ms (issue 57 % of cycles, 68-92 bytes of spills at 128 registers; 228-268 at
+// d = 2048, 128-144 at d = 8192), three primes with whole words and a separate
+// reconstruction took 13.
 #pragma once
 #include <cstdint>
 
